@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_query_batch(DevBox b, BatchScr
 
 __global__ void __launch_bounds__(kQueryThreads) k_translate(DevBox b, int slot, double vx, double vy, double vz) {
     __shared__ double refpos[3];
-    block_translate(b, slot, Vec3{vx, vy, vz}, refpos);
+    block_translate(b, slot, threadIdx.x == 0 ? vx : (threadIdx.x == 1 ? vy : vz), refpos);
 }
 
 __global__ void __launch_bounds__(kQueryThreads) k_merge(DevBox b, int ms, int os, int mslot, int oslot,
@@ -517,6 +517,7 @@ DevBox plan_fixed(const StateView &st) {
     b.L = st.box_length;
     b.n_div = st.n_div;
     b.step = double(st.n_div) / st.box_length;
+    b.step_f = float(b.step);
     b.n_cells = st.n_div * st.n_div * st.n_div;
     b.ns = st.ns;
     b.nslots = st.nslots;

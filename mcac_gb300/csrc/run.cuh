@@ -986,9 +986,8 @@ __device__ inline bool step_commit(const BoxRun &R, RS &sm, long long &t_phase) 
     const DevBox &b = R.box;
     RunState &st = *R.st;
     const int slot = sm.slot;
-    const Vec3 dir{sm.dir[0], sm.dir[1], sm.dir[2]};
     const int ms = sm.ms, os = sm.os, oslot = sm.oslot;
-    block_translate(b, slot, Vec3{dir.x * sm.move, dir.y * sm.move, dir.z * sm.move}, sm.refpos);
+    block_translate(b, slot, tid < 3 ? sm.dir[tid] * sm.move : 0.0, sm.refpos);
     if (tid == 0) {
         const long long t = clock64();
         st.cyc_move += t - t_phase;
