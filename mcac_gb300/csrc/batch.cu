@@ -13,6 +13,7 @@
 #include "host_box.hpp"
 #include "run.cuh"
 #include "spec.cuh"
+#include "step.cuh"
 
 namespace mcacg {
 
@@ -31,6 +32,8 @@ constexpr int kRunThreadChoices[] = {32, 64, 128, 256, 512};
 // an SM (shared memory being the limit there, not registers).
 template <int NT>
 using RunSmemFor = typename std::conditional<(NT <= 32), RunSmemSmall, RunSmem>::type;
+template <int NT>
+using LoopSmemFor = LoopSmemT<RunSmemFor<NT>>;
 // wall time of one launch when boxes run to their stop criteria
 constexpr long long kRunLaunchBudgetNs = 200LL * 1000 * 1000;
 
@@ -42,9 +45,8 @@ template <int NT>
 __global__ void __launch_bounds__(NT, 512 / NT) k_run(const BoxRun *runs, int n, long long max_steps,
                                                       long long budget_ns, const int *order) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    RunSmemFor<NT> &sm = *reinterpret_cast<RunSmemFor<NT> *>(smem_raw);
-    __shared__ __align__(16) BoxRun R;
-    __shared__ __align__(16) RunState st;  // the box's loop state, kept on chip for the launch
+    LoopSmemFor<NT> &sm = *reinterpret_cast<LoopSmemFor<NT> *>(smem_raw);
+    BoxRun &R = sm.R;
     if (int(blockIdx.x) >= n) return;
     const int box = order != nullptr ? order[blockIdx.x] : int(blockIdx.x);
     RunState *st_global = runs[box].st;
@@ -56,16 +58,17 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_run(const BoxRun *runs, int n,
         for (int k = threadIdx.x; k < words; k += NT) dst[k] = src[k];
         const int swords = int(sizeof(RunState) / sizeof(int));
         const int *ssrc = reinterpret_cast<const int *>(st_global);
-        int *sdst = reinterpret_cast<int *>(&st);
+        int *sdst = reinterpret_cast<int *>(&sm.st);
         for (int k = threadIdx.x; k < swords; k += NT) sdst[k] = ssrc[k];
     }
+    DevScalars *sc_global = runs[box].box.sc;
     __syncthreads();
     if (threadIdx.x == 0) {
-        R.st = &st;
+        R.st = &sm.st;
+        sm.sc = *sc_global;
+        R.box.sc = &sm.sc;
         // every step starts only before the deadline (a step is never cut)
         sm.deadline = budget_ns > 0 ? global_ns() + (unsigned long long)budget_ns : 0ULL;
-    }
-    if (threadIdx.x == 0) {
         sm.live.allow = decltype(sm.live)::kCap > 1 ? 1 : 0;
         sm.live.max = R.live_max;
         sm.live.on = 0;
@@ -73,14 +76,14 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_run(const BoxRun *runs, int n,
     __syncthreads();
     tree_cache_load(R, sm.tree);
     live_load(R, sm.live, sm.u.q.warp_tmp);
-    for (long long s = 0; s < max_steps; ++s)
-        if (!block_mc_step(R, sm)) break;
+    block_steps(sm, max_steps);
     __syncthreads();
     {
         const int swords = int(sizeof(RunState) / sizeof(int));
-        const int *ssrc = reinterpret_cast<const int *>(&st);
+        const int *ssrc = reinterpret_cast<const int *>(&sm.st);
         int *sdst = reinterpret_cast<int *>(st_global);
         for (int k = threadIdx.x; k < swords; k += NT) sdst[k] = ssrc[k];
+        if (threadIdx.x == 0) *sc_global = sm.sc;
     }
 }
 
@@ -262,7 +265,7 @@ bool ok_cuda(cudaError_t e, std::string *err, const char *what) {
 template <int NT>
 cudaError_t prepare_k_run() {
     cudaError_t e =
-        cudaFuncSetAttribute(k_run<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(RunSmemFor<NT>)));
+        cudaFuncSetAttribute(k_run<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(LoopSmemFor<NT>)));
     if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(k_run<NT>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
 }
@@ -278,11 +281,11 @@ cudaError_t prepare_all_k_run() {
 cudaError_t launch_k_run(int nt, int grid, cudaStream_t s, const BoxRun *runs, int n, long long steps,
                          long long budget_ns = 0, const int *order = nullptr) {
     switch (nt) {
-        case 32: k_run<32><<<grid, 32, sizeof(RunSmemFor<32>), s>>>(runs, n, steps, budget_ns, order); break;
-        case 64: k_run<64><<<grid, 64, sizeof(RunSmem), s>>>(runs, n, steps, budget_ns, order); break;
-        case 128: k_run<128><<<grid, 128, sizeof(RunSmem), s>>>(runs, n, steps, budget_ns, order); break;
-        case 512: k_run<512><<<grid, 512, sizeof(RunSmem), s>>>(runs, n, steps, budget_ns, order); break;
-        default: k_run<256><<<grid, 256, sizeof(RunSmem), s>>>(runs, n, steps, budget_ns, order); break;
+        case 32: k_run<32><<<grid, 32, sizeof(LoopSmemFor<32>), s>>>(runs, n, steps, budget_ns, order); break;
+        case 64: k_run<64><<<grid, 64, sizeof(LoopSmemFor<64>), s>>>(runs, n, steps, budget_ns, order); break;
+        case 128: k_run<128><<<grid, 128, sizeof(LoopSmemFor<128>), s>>>(runs, n, steps, budget_ns, order); break;
+        case 512: k_run<512><<<grid, 512, sizeof(LoopSmemFor<512>), s>>>(runs, n, steps, budget_ns, order); break;
+        default: k_run<256><<<grid, 256, sizeof(LoopSmemFor<256>), s>>>(runs, n, steps, budget_ns, order); break;
     }
     return cudaGetLastError();
 }
@@ -347,11 +350,11 @@ cudaError_t spec_clusters(int nt, int k, int *clusters) {
 int occupancy_k_run(int nt, int *per_sm) {
     cudaError_t e;
     switch (nt) {
-        case 32: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_run<32>, 32, sizeof(RunSmemFor<32>)); break;
-        case 64: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_run<64>, 64, sizeof(RunSmem)); break;
-        case 128: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_run<128>, 128, sizeof(RunSmem)); break;
-        case 512: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_run<512>, 512, sizeof(RunSmem)); break;
-        default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_run<256>, 256, sizeof(RunSmem)); break;
+        case 32: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_run<32>, 32, sizeof(LoopSmemFor<32>)); break;
+        case 64: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_run<64>, 64, sizeof(LoopSmemFor<64>)); break;
+        case 128: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_run<128>, 128, sizeof(LoopSmemFor<128>)); break;
+        case 512: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_run<512>, 512, sizeof(LoopSmemFor<512>)); break;
+        default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_run<256>, 256, sizeof(LoopSmemFor<256>)); break;
     }
     return e == cudaSuccess ? ST_OK : ST_CUDA;
 }
@@ -398,6 +401,12 @@ int make_box_run(const DevBox &b, const mcacg_params &p, double time, RunState *
                            p.with_surface_reactions ? p.u_sg : 0.0,
                            1.0 / p.gaz_mean_free_path,
                            1.0 / p.fractal_dimension,
+                           float(p.viscosity),
+                           float(p.gaz_mean_free_path),
+                           float(1.0 / p.gaz_mean_free_path),
+                           float(1.0 / p.fractal_dimension),
+                           float(p.density),
+                           float(p.temperature),
                            p.with_surface_reactions ? 1 : 0,
                            p.with_surface_reactions && p.individual_surf_reactions ? 1 : 0,
                            int(std::max<int64_t>(1, p.full_aggregate_update_frequency)),

@@ -256,6 +256,19 @@ __device__ __forceinline__ double wrap_position(double p, double L) {
     return dbits(p) >= 0 && dbits(p) < dbits(L) ? p : periodic_position_call(p, L);
 }
 
+// division and square root out of line: each inlined copy is some 20
+// instructions of a path that is run once a step
+static __device__ __noinline__ double fp64_div(double a, double b) { return a / b; }
+static __device__ __noinline__ double fp64_sqrt(double a) { return sqrt(a); }
+// verlet_coord clamped to the grid, from the FP32 coordinate xf: its product
+// with step_f is within 4 roundings of 2^-24 of n_div, so the floor is the
+// FP64 one further than 2e-6 n_div from an integer; else FP64 decides
+__device__ __forceinline__ int verlet_coord_dev(const DevBox &b, double x, float xf) {
+    const float q = xf * b.step_f, f = floorf(q), g = q - f, tol = 2e-6f * float(b.n_div);
+    const int c = g > tol && g < 1.f - tol && f < 1e6f ? int(f) : verlet_coord(x, b.step);
+    return min(max(c, 0), b.n_div - 1);
+}
+
 static __device__ __noinline__ double sweep_contact_general(Vec3 p1, double r1, Vec3 p2, double r2, Vec3 dir, double dist,
                                                      double L) {
     return sweep_contact_distance(p1, r1, p2, r2, dir, dist, L);
@@ -271,7 +284,8 @@ static __device__ __noinline__ double sweep_contact_general(Vec3 p1, double r1, 
 // and some twenty comparisons less). Together with the FP32 cell range:
 // 10 000 queries on a million spheres 782 -> 728 us, single queries 20.3 ->
 // 18.8 us, the 512-box ensemble's step 39.5 -> 35.8 us.
-__device__ inline double sweep_contact_fast(Vec3 p1, double r1, Vec3 p2, double r2, Vec3 dir, double dist, double L) {
+static __device__ __noinline__ double sweep_contact_fast(Vec3 p1, double r1, Vec3 p2, double r2, Vec3 dir, double dist,
+                                                         double L) {
     const double dc = r1 + r2;
     const double dc2 = dc * dc;
     {
@@ -316,7 +330,7 @@ __device__ inline double sweep_contact_fast(Vec3 p1, double r1, Vec3 p2, double 
     const double cz = d[0] * u[1] - d[1] * u[0];
     const double axis = cx * cx + cy * cy + cz * cz;
     if (!nonneg_le(axis, dc2)) return inf;
-    return proj - sqrt(dc2 - axis);
+    return proj - fp64_sqrt(dc2 - axis);
 }
 
 // Conservative FP32 capsule test: can a sphere at p2 (radius folded into
@@ -1186,6 +1200,14 @@ __device__ __forceinline__ int fine_index(float x, float step, int n) {
     if (!(f > -1e6f && f < 1e6f)) f = 0.f;
     return periodic_cell(static_cast<int>(f), n);
 }
+// The same for a coordinate in [0, n / step] (a wrapped position; rounding
+// may give n itself, the image of 0), without the modulo.
+__device__ __forceinline__ int fine_index_near(float x, float step, int n) {
+    const float f = floorf(x * step);
+    if (!(f >= 0.f && f <= float(n))) return fine_index(x, step, n);
+    const int i = static_cast<int>(f);
+    return i >= n ? 0 : i;
+}
 __device__ __forceinline__ int fine_cell_of(const DevBox &b, float x, float y, float z) {
     const int n = b.fine_div;
     return (fine_index(x, b.fine_step_f, n) * n + fine_index(y, b.fine_step_f, n)) * n +
@@ -1289,7 +1311,7 @@ __device__ inline void block_translate(const DevBox &b, int slot, double vl, dou
             A(b, AGG_X + tid, slot) = x;
             refpos_sm[tid] = x - A(b, AGG_RX + tid, slot);
             xf = float(x);
-            vc = min(max(verlet_coord(x, b.step), 0), b.n_div - 1);
+            vc = verlet_coord_dev(b, x, xf);
             if (b.fine_div > 0) fc = fine_index(xf, b.fine_step_f, b.fine_div);
         }
         const float yf = __shfl_sync(0xffffffffu, xf, 1), zf = __shfl_sync(0xffffffffu, xf, 2);

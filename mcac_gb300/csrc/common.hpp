@@ -13,9 +13,11 @@
 #if defined(__CUDACC__)
 #define MCACG_HD __host__ __device__ __forceinline__
 #define MCACG_UNROLL _Pragma("unroll")
+#define MCACG_NO_UNROLL _Pragma("unroll 1")  // a loop that almost never runs more than once
 #else
 #define MCACG_HD inline
 #define MCACG_UNROLL
+#define MCACG_NO_UNROLL
 #endif
 
 namespace mcacg {
@@ -55,14 +57,18 @@ constexpr int kWrapCap = 64;
 MCACG_HD double periodic_distance(double d, double dim) {
     double half = 0.5 * dim;
     int guard = 0;
+MCACG_NO_UNROLL
     while (d < -half && guard < kWrapCap) d += dim, ++guard;
+MCACG_NO_UNROLL
     while (d >= half && guard < kWrapCap) d -= dim, ++guard;
     if (guard >= kWrapCap) d = d - dim * floor(d / dim + 0.5);
     return d;
 }
 MCACG_HD double periodic_position(double p, double dim) {
     int guard = 0;
+MCACG_NO_UNROLL
     while (p < 0 && guard < kWrapCap) p += dim, ++guard;
+MCACG_NO_UNROLL
     while (p >= dim && guard < kWrapCap) p -= dim, ++guard;
     if (guard >= kWrapCap) p = p - dim * floor(p / dim);
     return p;
@@ -123,8 +129,11 @@ MCACG_UNROLL
         nper[l] = (np >= 0 && np <= 16) ? static_cast<int>(np) : (np > 16 ? 16 : 0);
     }
     double res = std::numeric_limits<double>::infinity();
+MCACG_NO_UNROLL
     for (int i = 0; i <= nper[0]; i++) {
+MCACG_NO_UNROLL
         for (int j = 0; j <= nper[1]; j++) {
+MCACG_NO_UNROLL
             for (int k = 0; k <= nper[2]; k++) {
                 double p3x = q[0] + i * L, p3y = q[1] + j * L, p3z = q[2] + k * L;
                 double dx = p3x - p1.x, dy = p3y - p1.y, dz = p3z - p1.z;

@@ -80,7 +80,7 @@ __device__ inline int block_scan_global(int *data, int n, int *warp_tmp) {
 
 // Move every live segment to the front of the other pool buffer, in slot
 // order. Uses counters[] and row_cnt[] as scratch.
-__device__ inline void block_compact_pool(const DevBox &b, int *warp_tmp) {
+static __device__ __noinline__ void block_compact_pool(const DevBox &b, int *warp_tmp) {
     DevScalars *sc = b.sc;
     const int from = sc->pool_sel, to = 1 - from;
     // prefix of member counts over slots, staged in row_cnt (size >= nslots+1)
@@ -249,6 +249,52 @@ __device__ inline void block_pair_scan(const DevBox &b, const int *mem, int n, S
         __syncthreads();
     }
     }  // all pairs: both branches end on a barrier
+}
+
+// The volume and surface corrections, out of line: boxes without them keep
+// the merge's code compact (the loop is bound by instruction fetch among
+// others).
+//
+// compute_volume_surface, "caps" (aggregat.cpp:358-388), one thread: each
+// sphere's contacts with later ones, in (i, j) order, take their caps off
+// both spheres; a sphere is clamped at 0 once its own contacts are done. The
+// reference visits a sphere's contacts in its hash map's order; here they go
+// by index.
+static __device__ __noinline__ void thread_merge_caps(const DevBox &b, const int *mem, int n, int P) {
+    double *wv = b.work;
+    const size_t W = size_t(b.ns);
+    for (int p = 0; p < P; ++p) {
+        const int i = b.pair_i[p], j = b.pair_j[p];
+        const int si = mem[i], sj = mem[j];
+        const SphereCaps k = sphere_caps(S(b, SPH_R, si), S(b, SPH_VOLUME, si), S(b, SPH_SURFACE, si),
+                                         S(b, SPH_R, sj), S(b, SPH_VOLUME, sj), S(b, SPH_SURFACE, sj), b.pair_d[p]);
+        wv[0 * W + i] = wv[0 * W + i] - k.v1;
+        wv[1 * W + i] = wv[1 * W + i] - k.s1;
+        wv[0 * W + j] = wv[0 * W + j] - k.v2;
+        wv[1 * W + j] = wv[1 * W + j] - k.s2;
+    }
+    // the clamps: a sphere's value is final once its row is done, and later
+    // rows never touch it
+    for (int i = 0; i < n; ++i) {
+        wv[0 * W + i] = dmax(wv[0 * W + i], 0.0);
+        wv[1 * W + i] = dmax(wv[1 * W + i], 0.0);
+    }
+}
+// "alphas" (aggregat.cpp:391-426), one thread: the sums over every contact
+// seen from both spheres (here each pair twice in a row, in (i, j) order),
+// then the corrections.
+static __device__ __noinline__ void alpha_add_call(AlphaSums &a, double r1, double r2, double d) {
+    alpha_add(a, r1, r2, d);
+}
+static __device__ __noinline__ void thread_merge_alphas(const DevBox &b, const int *mem, int n, int P, double *volume,
+                                                        double *surface, double *overlap, double *coord) {
+    AlphaSums a{0., 0., 0., 0., 0., 0.};
+    for (int p = 0; p < P; ++p) {
+        const double ri = S(b, SPH_R, mem[b.pair_i[p]]), rj = S(b, SPH_R, mem[b.pair_j[p]]);
+        alpha_add_call(a, ri, rj, b.pair_d[p]);
+        alpha_add_call(a, rj, ri, b.pair_d[p]);
+    }
+    alpha_finish(a, n, 2 * P, volume, surface, overlap, coord);
 }
 
 // AggregatList::merge + Aggregate::merge + Aggregate::update (geometry).
@@ -428,29 +474,7 @@ __device__ inline void block_merge(const DevBox &b, int ms, int os, int mslot, i
         wv[6 * W + k] = S(b, SPH_R, s);
     }
     __syncthreads();
-    if (b.volsurf == VS_CAPS && tid == 0) {
-        // compute_volume_surface, "caps" (aggregat.cpp:358-388): each
-        // sphere's contacts with later ones, in (i, j) order, take their caps
-        // off both spheres; a sphere is clamped at 0 once its own contacts
-        // are done. The reference visits a sphere's contacts in its hash
-        // map's order; here they go by index.
-        for (int p = 0; p < P; ++p) {
-            const int i = b.pair_i[p], j = b.pair_j[p];
-            const int si = mem[i], sj = mem[j];
-            const SphereCaps k = sphere_caps(S(b, SPH_R, si), S(b, SPH_VOLUME, si), S(b, SPH_SURFACE, si),
-                                             S(b, SPH_R, sj), S(b, SPH_VOLUME, sj), S(b, SPH_SURFACE, sj), b.pair_d[p]);
-            wv[0 * W + i] = wv[0 * W + i] - k.v1;
-            wv[1 * W + i] = wv[1 * W + i] - k.s1;
-            wv[0 * W + j] = wv[0 * W + j] - k.v2;
-            wv[1 * W + j] = wv[1 * W + j] - k.s2;
-        }
-        // the clamps: a sphere's value is final once its row is done, and
-        // later rows never touch it
-        for (int i = 0; i < n; ++i) {
-            wv[0 * W + i] = dmax(wv[0 * W + i], 0.0);
-            wv[1 * W + i] = dmax(wv[1 * W + i], 0.0);
-        }
-    }
+    if (b.volsurf == VS_CAPS && tid == 0) thread_merge_caps(b, mem, n, P);
     __syncthreads();
     for (int k = tid; k < n; k += NT) {
         const int s = mem[k];
@@ -499,18 +523,8 @@ __device__ inline void block_merge(const DevBox &b, int ms, int os, int mslot, i
             sm.overlap = sm.sums[7] / static_cast<double>(2 * P);
             sm.coord = static_cast<double>(2 * P) / static_cast<double>(n);
         }
-        if (b.volsurf == VS_ALPHAS) {
-            // compute_volume_surface, "alphas" (aggregat.cpp:391-426): the
-            // sums over every contact seen from both spheres (here each pair
-            // twice in a row, in (i, j) order), then the corrections
-            AlphaSums a{0., 0., 0., 0., 0., 0.};
-            for (int p = 0; p < P; ++p) {
-                const double ri = S(b, SPH_R, mem[b.pair_i[p]]), rj = S(b, SPH_R, mem[b.pair_j[p]]);
-                alpha_add(a, ri, rj, b.pair_d[p]);
-                alpha_add(a, rj, ri, b.pair_d[p]);
-            }
-            alpha_finish(a, n, 2 * P, &sm.sums[0], &sm.sums[1], &sm.overlap, &sm.coord);
-        }
+        if (b.volsurf == VS_ALPHAS)
+            thread_merge_alphas(b, mem, n, P, &sm.sums[0], &sm.sums[1], &sm.overlap, &sm.coord);
     }
     __syncthreads();
     const double V = sm.sums[0], Sf = sm.sums[1];
@@ -615,8 +629,8 @@ __device__ inline void block_merge(const DevBox &b, int ms, int os, int mslot, i
 // on the dynamics, are left to the merge and to the read-back unless
 // 'overlap' asks for them; "caps" and "alphas" need the pairs for the volume
 // and set them here.
-__device__ inline double thread_update_geometry(const DevBox &b, int a, bool full, double *vol_pp_out,
-                                                bool overlap = false) {
+static __device__ __noinline__ double thread_update_geometry(const DevBox &b, int a, bool full, double *vol_pp_out,
+                                                             bool overlap = false) {
     const int n = b.agg_n[a];
     const int *mem = b.pool_id[b.sc->pool_sel] + b.agg_off[a];
     double volume = A(b, AGG_VOLUME, a);
@@ -666,8 +680,8 @@ __device__ inline double thread_update_geometry(const DevBox &b, int a, bool ful
                     b.sph_volw[sj] = b.sph_volw[sj] - k.v2;
                     surf_w[sj] = surf_w[sj] - k.s2;
                 } else if (b.volsurf == VS_ALPHAS) {
-                    alpha_add(al, ri, rj, dist);
-                    alpha_add(al, rj, ri, dist);
+                    alpha_add_call(al, ri, rj, dist);
+                    alpha_add_call(al, rj, ri, dist);
                 }
             }
             if (b.volsurf == VS_CAPS) {

@@ -31,6 +31,8 @@ struct PhysParams {
     double viscosity, lambda, fractal_dimension, density, temperature;
     double u_sg;        // surface growth velocity dr/dt (m/s)
     double inv_lambda, inv_fractal_dimension;
+    // the same rounded to FP32, as the loop's physics uses them
+    float viscosity_f, lambda_f, inv_lambda_f, inv_fractal_dimension_f, density_f, temperature_f;
     int growth;         // with_surface_reactions
     int individual;     // individual_surf_reactions: only the moved aggregate grows and is updated
     int full_update_every;  // full_aggregate_update_frequency
@@ -112,11 +114,47 @@ using TreeCacheLarge = TreeCacheT<640>;
 constexpr unsigned long long kTreeHeadroom = 1ULL << 62;
 
 
+// Limits of the steps that one warp runs by itself (step.cuh); what is larger
+// goes to the block.
+constexpr int kWarpCells = 128;   // cells a query visits (four per lane)
+constexpr int kWarpQueue = 256;   // aggregates listed for a query
+constexpr int kWarpCands = 32;    // neighbours past the FP32 screen; sphere pairs to refine
+constexpr int kWarpPairs = 1024;  // sphere pairs screened
+constexpr int kWarpMove = 64;     // spheres translated (no limit where a block is one warp)
+
+// Scratch of a one-warp step.
+struct WarpScratch {
+    int queue[kWarpQueue];
+    // neighbours past the FP32 screen, with their scan keys
+    int scr_slot[kWarpCands];
+    long long scr_key[kWarpCands];
+    // candidates as found, and in filter order (distances as ordered keys)
+    unsigned long long c_db[kWarpCands];
+    long long c_key[kWarpCands];
+    int c_slot[kWarpCands];
+    unsigned long long s_db[kWarpCands];
+    int s_slot[kWarpCands], s_off[kWarpCands], s_pre[kWarpCands];
+    // sphere pairs to refine
+    unsigned long long p_key[kWarpCands], p_ij[kWarpCands];
+    int p_r[kWarpCands], p_si[kWarpCands], p_sj[kWarpCands];
+};
+
+// Scratch of a one-warp merge (at most 32 spheres, 496 pairs). Rows of 33, so
+// that lanes reading one row each meet different banks.
+struct WarpMergeScratch {
+    double rel[3][33];
+    double term[8][33];
+    double ov[496];
+    unsigned short pair[496];  // i << 8 | j
+};
+
 template <class QS, class MS, class TC, class LL>
 struct RunSmemT {
     union {
         QS q;
         MS m;
+        WarpScratch w;
+        WarpMergeScratch wm;
     } u;
     MergeOut mout;
     double refpos[3];
@@ -127,6 +165,8 @@ struct RunSmemT {
     int slot, contact, stop, merged, rescale;
     int keep, removed;
     int ms, os, oslot;  // contact of this step: spheres and the other slot
+    int op;             // what warp 0 asks the block to do (step.cuh)
+    int try_merge, mslot, cslot;  // a merge is due, of these two slots
     unsigned long long tree_tmp;  // block reduction scratch
     double step_dt;               // this step's time increment
     double dt_indiv, step_dt_indiv;  // the moved aggregate's own time step, and its increment
@@ -142,7 +182,7 @@ using RunSmemSmall = RunSmemT<QuerySmemSmall, MergeSmemSmall, TreeCache, LiveLis
 // ------------------------------------------------------------ sum tree
 // Marks the kept levels and copies them (all threads).
 template <class TC>
-__device__ inline void tree_cache_load(const BoxRun &R, TC &c) {
+__device__ __noinline__ void tree_cache_load(const BoxRun &R, TC &c) {
     if (threadIdx.x == 0) {
         int used = 0;
         for (int lev = kMaxTreeLevels - 1; lev >= 0; --lev) c.coff[lev] = -1;
@@ -160,30 +200,38 @@ __device__ inline void tree_cache_load(const BoxRun &R, TC &c) {
     __syncthreads();
 }
 
+// Warp 0: the weights of the (up to) 32 nodes of level 'lev' from 'base' on,
+// one per lane (0 beyond the level).
+template <class TC>
+__device__ __forceinline__ unsigned long long tree_children(const BoxRun &R, const TC &c, int lev, int base) {
+    const int k = base + (threadIdx.x & 31), co = c.coff[lev];
+    if (k >= R.tree_len[lev]) return 0ULL;
+    return co >= 0 ? c.v[co + k] : R.tree[R.tree_off[lev] + k];
+}
+// Warp 0: which of the lanes' weights holds the target 't' (in lane order);
+// t becomes the target within it.
+__device__ __forceinline__ int tree_pick_child(unsigned long long v, unsigned long long &t) {
+    const int lane = threadIdx.x & 31;
+    unsigned long long incl = v;  // inclusive scan over the 32 children
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    const unsigned over = __ballot_sync(0xffffffffu, incl > t && v > 0ULL);
+    const unsigned nonzero = __ballot_sync(0xffffffffu, v > 0ULL);
+    const int pick = over ? __ffs(over) - 1 : (nonzero ? 31 - __clz(nonzero) : 0);
+    t -= __shfl_sync(0xffffffffu, incl - v, pick);
+    return pick;
+}
 // Warp 0: descend from the top level to a leaf holding the target 't'
 // (0 <= t < total).
 template <class TC>
 __device__ inline int tree_sample(const BoxRun &R, const TC &c, unsigned long long t) {
-    const int lane = threadIdx.x & 31;
     int node = 0;  // index within the current level
     for (int lev = R.tree_levels - 1; lev >= 0; --lev) {
         const int base = node * kTreeFan;
-        const int len = R.tree_len[lev];
-        const int co = c.coff[lev];
-        const unsigned long long v =
-            (base + lane < len) ? (co >= 0 ? c.v[co + base + lane] : R.tree[R.tree_off[lev] + base + lane]) : 0ULL;
-        // inclusive scan over the 32 children (fixed order)
-        unsigned long long incl = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        const unsigned over = __ballot_sync(0xffffffffu, incl > t && v > 0ULL);
-        const unsigned nonzero = __ballot_sync(0xffffffffu, v > 0ULL);
-        const int pick = over ? __ffs(over) - 1 : (nonzero ? 31 - __clz(nonzero) : 0);
-        t -= __shfl_sync(0xffffffffu, incl - v, pick);
-        node = base + pick;
+        node = base + tree_pick_child(tree_children(R, c, lev, base), t);
     }
     return node;
 }
@@ -276,7 +324,7 @@ __device__ __forceinline__ void tree_total_to_state(RunState &st, unsigned long 
 // weights when at most live.max aggregates are left (all threads); turns it
 // off otherwise. The pick and the query then read the list.
 template <class LL>
-__device__ inline void live_load(const BoxRun &R, LL &L, int *warp_tmp) {
+__device__ __noinline__ void live_load(const BoxRun &R, LL &L, int *warp_tmp) {
     const DevBox &b = R.box;
     const int tid = threadIdx.x, NT = blockDim.x;
     const int n_alive = b.sc->n_alive;
@@ -361,6 +409,35 @@ __device__ inline void live_merge(LL &L, int keep, int removed, unsigned long lo
     L.n = j;
 }
 
+// live_merge by warp 0: the entries after the removed one move down a place.
+template <class LL>
+__device__ inline void warp_live_merge(LL &L, int keep, int removed, unsigned long long w_keep) {
+    static_assert(LL::kCap <= 128, "four entries a lane");
+    const int lane = threadIdx.x & 31, n = L.n;
+    int s[4], gone = n;
+    unsigned long long w[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int i = 32 * u + lane;
+        s[u] = i < n ? L.slot[i] : -1;
+        w[u] = i < n ? (s[u] == keep ? w_keep : L.w[i]) : 0ULL;
+        const unsigned m = __ballot_sync(0xffffffffu, s[u] == removed && i < n);
+        if (m != 0u) gone = 32 * u + __ffs(m) - 1;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int i = 32 * u + lane;
+        if (i < n && i != gone) {
+            const int j = i - (i > gone ? 1 : 0);
+            L.slot[j] = s[u];
+            L.w[j] = w[u];
+        }
+    }
+    if (lane == 0 && gone < n) L.n = n - 1;
+    __syncwarp();
+}
+
 // ------------------------------------------------------------ physics
 // update_partial's physics (aggregat.cpp:264-276, physical_model.cpp:550-617):
 // friction, mobility diameter, time step and mean free path, in FP32 with
@@ -373,26 +450,31 @@ __device__ inline void live_merge(LL &L, int keep, int removed, unsigned long lo
 // ~1e-9..1e-2 s). The common factors are taken once: one pow (its square
 // root form squared) and the reciprocals of the gas mean free path and of
 // the fractal dimension from the host. dg/dp, a geometric ratio, stays FP64.
-__device__ inline void device_physics(const PhysParams &p, double V, double vol_pp, double dp, double rg, double *f_agg,
-                               double *d_m, double *time_step, double *lpm, double *dg_over_dp) {
-    const float r = float(0.5 * dp);
+// Returns (f, d_m, time step, lpm) from the mean radius, the volume and the
+// mean sphere volume.
+static __device__ __noinline__ float4 physics_f32(const PhysParams &p, float r, float V, float vol_pp) {
     const float a = 1.142f, b = 0.558f, c = 0.999f;
-    const float lambda = float(p.lambda), inv_lambda = float(p.inv_lambda);
+    const float lambda = p.lambda_f, inv_lambda = p.inv_lambda_f;
     const float lr = lambda / r;
     const float fe = 0.689f * (1.f + erff((lr + 4.454f) * (1.f / 10.628f)));
     const float cc = 1.f + lr * (a + b * expf(-c * r * inv_lambda));
-    const float ratio = float(V) / float(vol_pp);
-    const float pw2 = powf(ratio, 0.5f * fe * float(p.inv_fractal_dimension));
+    const float ratio = V / vol_pp;
+    const float pw2 = powf(ratio, 0.5f * fe * p.inv_fractal_dimension_f);
     const float pw = pw2 * pw2;
-    const float f = (6.f * float(pi_value()) * float(p.viscosity) * r / cc) * pw;
+    const float f = (6.f * float(pi_value()) * p.viscosity_f * r / cc) * pw;
     const float ar = r * pw2;
     const float cc_a = 1.f + (lambda / ar) * (a + b * expf(-c * ar * inv_lambda));
-    const float ts = 3.f * (float(p.density) * float(V)) / f;
-    *f_agg = double(f);
-    *d_m = double((cc_a / cc) * 2.f * r * pw);
-    *time_step = double(ts);
-    *lpm = double(sqrtf(6.f * float(kBoltzmann) * float(p.temperature) / f * ts));
-    *dg_over_dp = rg / (0.5 * dp);
+    const float ts = 3.f * (p.density_f * V) / f;
+    return make_float4(f, (cc_a / cc) * 2.f * r * pw, ts, sqrtf(6.f * float(kBoltzmann) * p.temperature_f / f * ts));
+}
+__device__ inline void device_physics(const PhysParams &p, double V, double vol_pp, double dp, double rg, double *f_agg,
+                                      double *d_m, double *time_step, double *lpm, double *dg_over_dp) {
+    const float4 v = physics_f32(p, float(0.5 * dp), float(V), float(vol_pp));
+    *f_agg = double(v.x);
+    *d_m = double(v.y);
+    *time_step = double(v.z);
+    *lpm = double(v.w);
+    *dg_over_dp = fp64_div(rg, 0.5 * dp);
 }
 
 __device__ __forceinline__ bool run_finished(const BoxRun &R, const RunState &st, int n_alive) {
@@ -408,8 +490,6 @@ __device__ __forceinline__ bool run_finished(const BoxRun &R, const RunState &st
     return false;
 }
 
-// One MC step of one box by the whole block. Returns false when the box is
-// finished or in error (then nothing was done).
 // ------------------------------------------------------ surface growth
 // Sphere::croissance_surface (sphere.cpp:113-120) for every sphere of the box:
 // r += u_sg dt, volume and surface from the new radius. Each sphere is found
@@ -464,7 +544,7 @@ __device__ inline void block_grow_slot(const BoxRun &R, int slot, double dt) {
 // Aggregate::update / update_partial (aggregat.cpp:247-288) of one slot by
 // one thread: the geometry (thread_update_geometry), then the physics fields
 // in FP32 (device_physics). Returns r_max.
-__device__ inline double thread_update_aggregate(const BoxRun &R, int a, bool full) {
+static __device__ __noinline__ double thread_update_aggregate(const BoxRun &R, int a, bool full) {
     const DevBox &b = R.box;
     double vol_pp = 0.0;
     const double rmax = thread_update_geometry(b, a, full, &vol_pp);
@@ -482,7 +562,7 @@ __device__ inline double thread_update_aggregate(const BoxRun &R, int a, bool fu
 // the live count, leaves of the live slots (0 elsewhere), then each level
 // from the one below, and the total into the loop state. The FP64 weights
 // sit in the leaves (as bits) between the two passes.
-__device__ inline void block_tree_build(const BoxRun &R) {
+static __device__ __noinline__ void block_tree_build(const BoxRun &R) {
     const DevBox &b = R.box;
     const int tid = threadIdx.x, NT = blockDim.x;
     __shared__ unsigned long long max_bits;
@@ -975,6 +1055,118 @@ __device__ inline void apply_query(RunState &st, RS &sm, const QueryOut &q) {
     st.cyc_qpairs += q.cyc_pairs;
 }
 
+// Surface reactions before the merge (calcul.cpp:157-172), all threads:
+// growth or oxidation of every aggregate or of the moved one; sm.try_merge,
+// sm.mslot and sm.cslot are the merge that is still due.
+template <class RS>
+__device__ __noinline__ void commit_reactions(const BoxRun &R, RS &sm) {
+    const int tid = threadIdx.x;
+    const DevBox &b = R.box;
+    RunState &st = *R.st;
+    if (R.phys.individual)
+        block_grow_slot(R, sm.slot, sm.step_dt_indiv);
+    else
+        block_grow_spheres(R, sm.step_dt);
+    __syncthreads();
+    if (!R.phys.oxidation) return;
+    block_oxidize(R, sm, R.phys.individual ? sm.slot : -1);
+    if (tid == 0) {
+        if (b.sc->status != ST_OK) {
+            st.status = b.sc->status;
+            sm.stop = 1;
+        } else if (sm.try_merge) {
+            // AggregatList::merge takes the two spheres where they are now,
+            // and merges nothing when one is gone or they no longer touch
+            // (aggregat_list.cpp:367-378); the individual mode merges nothing
+            // after a split or a disappearance (calcul.cpp:173-178)
+            sm.mslot = b.sph_slot[sm.ms];
+            sm.cslot = b.sph_slot[sm.os];
+            if (sm.mslot < 0 || sm.cslot < 0 || sm.mslot == sm.cslot) sm.try_merge = 0;
+            if (R.phys.individual && (sm.split || sm.disappear)) sm.try_merge = 0;
+        }
+    }
+    __syncthreads();
+}
+
+// The merge of the step's contact (all threads): geometry, physics and, where
+// no growth rebuilds it anyway, the pick tree and the live list. An error
+// sets sm.stop.
+template <class RS>
+__device__ inline void commit_merge(const BoxRun &R, RS &sm) {
+    const int tid = threadIdx.x;
+    const DevBox &b = R.box;
+    RunState &st = *R.st;
+    block_merge(b, sm.ms, sm.os, sm.mslot, sm.cslot, sm.u.m, &sm.mout);
+    if (tid == 0) {
+        if (sm.mout.status != ST_OK) {
+            st.status = sm.mout.status;
+            sm.stop = 1;
+        } else if (sm.mout.merged) {
+            const int keep = sm.mout.keep, removed = sm.mout.removed;
+            double f, dm, ts, lpm, dgdp;
+            device_physics(R.phys, sm.mout.fields[AGG_VOLUME], sm.mout.vol_pp, sm.mout.fields[AGG_DP],
+                           sm.mout.fields[AGG_RG], &f, &dm, &ts, &lpm, &dgdp);
+            A(b, AGG_F_AGG, keep) = f;
+            A(b, AGG_D_M, keep) = dm;
+            A(b, AGG_TIME_STEP, keep) = ts;
+            A(b, AGG_LPM, keep) = lpm;
+            A(b, AGG_DG_OVER_DP, keep) = dgdp;
+            A(b, AGG_TIME, keep) = A(b, AGG_TIME, keep) + A(b, AGG_TIME, removed) - st.time;
+            sm.merged = 1;
+            sm.keep = keep;
+            sm.removed = removed;
+            st.c_merged_spheres += sm.mout.n;
+            st.c_merge_pairs += sm.mout.n_pairs;
+        }
+    }
+    __syncthreads();
+    if (sm.stop || !sm.merged || R.phys.growth) return;
+    if (tid < 32) {
+        tree_set(R, sm.tree, sm.removed, 0ULL);
+        const unsigned long long wk = tree_weight(st, A(b, AGG_TIME_STEP, sm.keep));
+        const unsigned long long total = tree_set(R, sm.tree, sm.keep, wk);
+        if (tid == 0) {
+            tree_total_to_state(st, total);
+            sm.rescale = total > kTreeHeadroom;  // a new scale keeps the total clear of 2^64
+            if (sm.live.on) live_merge(sm.live, sm.keep, sm.removed, wk);
+        }
+    }
+    __syncthreads();
+    if (sm.rescale) {
+        block_tree_build(R);
+        tree_cache_load(R, sm.tree);
+        live_load(R, sm.live, sm.u.q.warp_tmp);  // every weight changed
+    } else if (!sm.live.on && sm.live.allow && b.sc->n_alive <= sm.live.max) {
+        live_load(R, sm.live, sm.u.q.warp_tmp);  // few enough left now
+    }
+}
+
+// The update after growth and merge (all threads): update() on every
+// full_aggregate_update_frequency-th step without event, else
+// update_partial() (calcul.cpp:180-206), of every aggregate; in the
+// individual mode only of the moved one, unless there was an event.
+template <class RS>
+__device__ __noinline__ void commit_update(const BoxRun &R, RS &sm) {
+    const long long every = R.phys.full_update_every > 0 ? R.phys.full_update_every : 1;
+    const bool full = R.st->n_iter_without_event % every == 0;
+    const bool event = sm.merged || (R.phys.oxidation && (sm.split || sm.disappear));
+    block_update_one_or_all(R, sm, !R.phys.individual || event ? -1 : sm.slot, full);
+}
+
+// The end of a step (one thread): counters and stop criteria.
+template <class RS>
+__device__ __forceinline__ void step_end(const BoxRun &R, RS &sm) {
+    RunState &st = *R.st;
+    st.steps += 1;
+    if (sm.merged || (R.phys.oxidation && (sm.split || sm.disappear))) {
+        st.events += 1;
+        st.n_iter_without_event = 0;
+    } else {
+        st.n_iter_without_event += 1;
+    }
+    if (run_finished(R, st, R.box.sc->n_alive)) st.finished = 1;
+}
+
 // The rest of a step once its pick (sm.slot, sm.dir, sm.dt, sm.full,
 // sm.dt_indiv) and its query's answer (sm.contact, sm.move, sm.ms, sm.os,
 // sm.oslot) are known: translation, time, surface reactions, merge, pick
@@ -986,7 +1178,6 @@ __device__ inline bool step_commit(const BoxRun &R, RS &sm, long long &t_phase) 
     const DevBox &b = R.box;
     RunState &st = *R.st;
     const int slot = sm.slot;
-    const int ms = sm.ms, os = sm.os, oslot = sm.oslot;
     block_translate(b, slot, tid < 3 ? sm.dir[tid] * sm.move : 0.0, sm.refpos);
     if (tid == 0) {
         const long long t = clock64();
@@ -999,172 +1190,29 @@ __device__ inline bool step_commit(const BoxRun &R, RS &sm, long long &t_phase) 
         sm.merged = 0;
         sm.step_dt = dt;
         sm.step_dt_indiv = sm.contact ? sm.dt_indiv * (sm.move / sm.full + 0.0) : sm.dt_indiv;
+        sm.try_merge = sm.contact;
+        sm.mslot = slot;
+        sm.cslot = sm.oslot;
     }
     __syncthreads();
-    // surface reactions before the merge (calcul.cpp:157-172)
     if (R.phys.growth) {
-        if (R.phys.individual)
-            block_grow_slot(R, slot, sm.step_dt_indiv);
-        else
-            block_grow_spheres(R, sm.step_dt);
-    }
-    __syncthreads();
-    bool try_merge = sm.contact;
-    int mslot = slot, cslot = oslot;
-    if (R.phys.oxidation) {
-        block_oxidize(R, sm, R.phys.individual ? slot : -1);
-        if (tid == 0 && b.sc->status != ST_OK) {
-            st.status = b.sc->status;
-            sm.stop = 1;
-        }
-        __syncthreads();
+        commit_reactions(R, sm);
         if (sm.stop) return false;
-        // AggregatList::merge takes the two spheres where they are now, and
-        // merges nothing when one is gone or they no longer touch
-        // (aggregat_list.cpp:367-378); the individual mode merges nothing
-        // after a split or a disappearance (calcul.cpp:173-178)
-        if (try_merge) {
-            mslot = b.sph_slot[ms];
-            cslot = b.sph_slot[os];
-            if (mslot < 0 || cslot < 0 || mslot == cslot) try_merge = false;
-            if (R.phys.individual && (sm.split || sm.disappear)) try_merge = false;
-        }
     }
-    if (try_merge) {
-        block_merge(b, ms, os, mslot, cslot, sm.u.m, &sm.mout);
-        if (tid == 0) {
-            if (sm.mout.status != ST_OK) {
-                st.status = sm.mout.status;
-                sm.stop = 1;
-            } else if (sm.mout.merged) {
-                const int keep = sm.mout.keep, removed = sm.mout.removed;
-                double f, dm, ts, lpm, dgdp;
-                device_physics(R.phys, sm.mout.fields[AGG_VOLUME], sm.mout.vol_pp, sm.mout.fields[AGG_DP],
-                               sm.mout.fields[AGG_RG], &f, &dm, &ts, &lpm, &dgdp);
-                A(b, AGG_F_AGG, keep) = f;
-                A(b, AGG_D_M, keep) = dm;
-                A(b, AGG_TIME_STEP, keep) = ts;
-                A(b, AGG_LPM, keep) = lpm;
-                A(b, AGG_DG_OVER_DP, keep) = dgdp;
-                A(b, AGG_TIME, keep) = A(b, AGG_TIME, keep) + A(b, AGG_TIME, removed) - st.time;
-                sm.merged = 1;
-                sm.keep = keep;
-                sm.removed = removed;
-                st.c_merged_spheres += sm.mout.n;
-                st.c_merge_pairs += sm.mout.n_pairs;
-            }
-        }
-        __syncthreads();
+    if (sm.try_merge) {
+        commit_merge(R, sm);
         if (sm.stop) return false;
-        if (sm.merged && tid < 32 && !R.phys.growth) {
-            tree_set(R, sm.tree, sm.removed, 0ULL);
-            const unsigned long long wk = tree_weight(st, A(b, AGG_TIME_STEP, sm.keep));
-            const unsigned long long total = tree_set(R, sm.tree, sm.keep, wk);
-            if (tid == 0) {
-                tree_total_to_state(st, total);
-                sm.rescale = total > kTreeHeadroom;  // a new scale keeps the total clear of 2^64
-                if (sm.live.on) live_merge(sm.live, sm.keep, sm.removed, wk);
-            }
-        }
-        __syncthreads();
-        if (sm.merged && !R.phys.growth && sm.rescale) {
-            block_tree_build(R);
-            tree_cache_load(R, sm.tree);
-            live_load(R, sm.live, sm.u.q.warp_tmp);  // every weight changed
-        } else if (sm.merged && !R.phys.growth && !sm.live.on && sm.live.allow &&
-                   b.sc->n_alive <= sm.live.max) {
-            live_load(R, sm.live, sm.u.q.warp_tmp);  // few enough left now
-        }
     }
     if (R.phys.growth) {
-        // every aggregate after growth (and merge): update() on every
-        // full_aggregate_update_frequency-th step without event, else
-        // update_partial() (calcul.cpp:180-206); in the individual mode only
-        // the moved aggregate, unless there was a merge
         __syncthreads();
-        const long long every = R.phys.full_update_every > 0 ? R.phys.full_update_every : 1;
-        const bool full = st.n_iter_without_event % every == 0;
-        const bool event = sm.merged || (R.phys.oxidation && (sm.split || sm.disappear));
-        if (!R.phys.individual || event)
-            block_update_one_or_all(R, sm, -1, full);
-        else
-            block_update_one_or_all(R, sm, slot, full);
+        commit_update(R, sm);
     }
     if (tid == 0) {
         st.cyc_merge += clock64() - t_phase;
-        st.steps += 1;
-        if (sm.merged || (R.phys.oxidation && (sm.split || sm.disappear))) {
-            st.events += 1;
-            st.n_iter_without_event = 0;
-        } else {
-            st.n_iter_without_event += 1;
-        }
-        if (run_finished(R, st, b.sc->n_alive)) st.finished = 1;
+        step_end(R, sm);
     }
     __syncthreads();
     return true;
-}
-
-// One MC step of one box by the whole block. Returns false when the box is
-// finished or in error (then nothing was done).
-template <class RS>
-__device__ inline bool block_mc_step(const BoxRun &R, RS &sm) {
-    const int tid = threadIdx.x;
-    const DevBox &b = R.box;
-    RunState &st = *R.st;
-    long long t_phase = 0;
-    if (tid == 0) {
-        t_phase = clock64();
-        sm.stop = st.finished || st.status != ST_OK;
-        if (!sm.stop && run_finished(R, st, b.sc->n_alive)) {
-            st.finished = 1;
-            sm.stop = 1;
-        }
-        // a time-capped launch: checked before every step, so that a box of
-        // expensive steps does not hold the launch (and the other boxes,
-        // which wait for it) past the cap
-        if (!sm.stop && sm.deadline != 0ULL && global_ns() >= sm.deadline) sm.stop = 1;
-        if (!sm.stop) sm.t_pick = pick_target(st.rng, st.tree_total);
-    }
-    __syncthreads();
-    if (sm.stop) return false;
-    if (tid < 32) {
-        int slot = sm.live.on ? live_sample(sm.live, sm.t_pick) : tree_sample(R, sm.tree, sm.t_pick);
-        if (tid == 0) {
-            if (slot < 0 || slot >= b.nslots || b.agg_n[slot] == 0) {
-                st.status = ST_UNKNOWN;  // the tree lost a live slot: stop this box
-                sm.stop = 1;
-                slot = 0;
-            }
-            sm.slot = slot;
-            sm.dt = st.inv_weight;
-            sm.full = A(b, AGG_LPM, slot);
-            sm.dt_indiv = A(b, AGG_TIME_STEP, slot);
-            draw_direction(st.rng, sm.dir);
-        }
-    }
-    __syncthreads();
-    if (sm.stop) return false;
-    if (tid == 0) {
-        const long long t = clock64();
-        st.cyc_pick += t - t_phase;
-        t_phase = t;
-    }
-    if (R.lim.with_collisions) {
-        block_query(b, sm.slot, Vec3{sm.dir[0], sm.dir[1], sm.dir[2]}, sm.full, sm.u.q, &sm.live);
-        if (tid == 0) apply_query(st, sm, sm.u.q.out);
-    } else if (tid == 0) {
-        sm.contact = 0;
-        sm.move = sm.full;
-    }
-    __syncthreads();
-    if (sm.stop) return false;
-    if (tid == 0) {
-        const long long t = clock64();
-        st.cyc_query += t - t_phase;
-        t_phase = t;
-    }
-    return step_commit(R, sm, t_phase);
 }
 
 }  // namespace mcacg

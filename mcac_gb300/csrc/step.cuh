@@ -1,0 +1,1243 @@
+// MC steps of the device loop by one warp.
+//
+// Most steps of a run are small: an aggregate of a few spheres moves, a
+// handful of neighbours lie in its reach, and usually none is hit. Such a
+// step is a chain of short dependent operations -- loads that wait for one
+// another, FP64 instructions at 64 cycles each, barriers -- so it takes the
+// same time on 512 threads as on 32, and the barriers and the other warps'
+// copies of the uniform FP64 work come on top. Here warp 0 runs the whole
+// step alone, without a block barrier:
+//
+//   pick    the tree descent; the direction's FP64 work fills the wait for
+//           the tree's leaves;
+//   record  every field of the picked slot in one round of loads (lane f
+//           reads field f of the FP64 table and of the integer tables), and
+//           the members' relative positions behind it, used after the query;
+//   query   the same neighbours, filter, pairs and walk as block_query: the
+//           neighbours come through a queue in shared memory, so that a
+//           round of loads serves 32 list entries; a swept test takes three
+//           lanes, one axis each (warp_sweep, ~40 FP64 instructions for up
+//           to ten tests at once);
+//   move    member positions, three lanes a sphere;
+//   merge   up to 32 spheres, one per lane (warp_merge).
+//
+// Whatever is larger (long neighbour lists, many sphere pairs, aggregates of
+// many spheres, surface reactions, tree rebuilds) goes to the
+// block's routines: warp_steps returns the operation, all threads run it
+// (block_op), and warp 0 goes on from there. Both ways give the same bits.
+//
+// What bounds it: about 2000 warp instructions a step in one dependent
+// chain (9.5 cycles each on a box alone: 2.7 fixed latency, 3.0 waiting for
+// L2, 1.7 for FP64 and shared memory). Measured against the block's loop:
+// one box of 4096 monomers 15.4 -> 8.6 us a step; 2000 boxes of 1000
+// monomers, a warp each, 35.6 -> 17.5 us; the 512-box ensemble's 4000 early
+// steps 158 -> 97 ms; 48 served runs 559 -> 390 ms. The limits (kWarp*, in
+// run.cuh) lie where a warp's rounds over the work cost about what the
+// block's barriers and set-up do: four rounds of cells, two of members,
+// thirty-two of pair screens at two instructions a cycle.
+#pragma once
+#include "run.cuh"
+
+namespace mcacg {
+
+// What warp_steps asks the block to do.
+enum StepOp : int { STEP_EXIT, STEP_QUERY, STEP_MOVE, STEP_REACT, STEP_MERGE, STEP_TREE, STEP_LIVE, STEP_UPDATE };
+// Where warp 0 goes on.
+enum StepPhase : int { PH_START, PH_QUERIED, PH_MOVED, PH_REACTED, PH_MERGED, PH_END };
+
+__device__ __forceinline__ double shfl_d(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+__device__ __forceinline__ int shfl_i(int v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+__device__ __forceinline__ float shfl_f(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+__device__ __forceinline__ unsigned clock_lo() { return static_cast<unsigned>(clock()); }
+__device__ __forceinline__ unsigned lanes_below(int lane) { return (1u << lane) - 1u; }
+
+// x + y + z in that order, from the three lanes of a group whose first lane is g
+__device__ __forceinline__ double sum3(double v, int g) {
+    const double x = shfl_d(v, g), y = shfl_d(v, g + 1), z = shfl_d(v, g + 2);
+    return (x + y) + z;
+}
+
+// sweep_contact_fast by three lanes, one axis each: lane g + ax of a group
+// holds the two positions' coordinate ax (pa, pb); the direction's are on
+// lanes 0-2 (u). The result is valid on every lane of the group. All lanes
+// of the warp call it.
+__device__ inline double warp_sweep(int g, int ax, double pa, double pb, double r1, double r2, double u, double dist,
+                                    double L) {
+    const double dc = r1 + r2;
+    const double dc2 = dc * dc;
+    const double ua = shfl_d(u, ax), u1 = shfl_d(u, ax == 2 ? 0 : ax + 1), u2 = shfl_d(u, ax == 0 ? 2 : ax - 1);
+    const double d0 = wrap_distance(pa - pb, L);
+    const bool touch = nonneg_le(sum3(d0 * d0, g), dc2);
+    const double td = ua * dist;
+    const double moved = pa + td;
+    const bool back = dbits(td) < 0;
+    const double base = (back ? moved : pa) - dc;
+    const double end = (back ? pa : moved) + dc;
+    const double zone = end - base;
+    bool usual = abs_lt(zone, L);
+    double w = pb - base;
+    if (!abs_lt(w, L)) {
+        // fmod(w, L) for L <= |w| < 2 L: one exact subtraction
+        usual = usual && (dbits(w) & 0x7fffffffffffffffLL) < dbits(L) + (1LL << 52);
+        w = dbits(w) < 0 ? w + L : w - L;
+    }
+    if (neg(w)) w += L;
+    const double q = w + base;
+    const double d = q - pa;
+    const bool outside = (dbits(d) & 0x7fffffffffffffffLL) > dbits(zone);
+    const double e = moved - q;
+    const double proj = sum3(d * ua, g);
+    const double e2 = sum3(e * e, g);
+    const double d1 = shfl_d(d, ax == 2 ? g : g + ax + 1), d2 = shfl_d(d, ax == 0 ? g + 2 : g + ax - 1);
+    const double c = d1 * u2 - d2 * u1;
+    const double axis = sum3(c * c, g);
+    const unsigned unusual3 = (__ballot_sync(0xffffffffu, !usual) >> g) & 7u;
+    const unsigned outside3 = (__ballot_sync(0xffffffffu, outside) >> g) & 7u;
+    double res = CUDART_INF;
+    if (unusual3 == 0u && outside3 == 0u && !neg(proj) && nonneg_le(axis, dc2) &&
+        (nonneg_le(e2, dc2) || !(dkey(dist) < dkey(proj))))
+        res = proj - fp64_sqrt(dc2 - axis);
+    const unsigned any = __ballot_sync(0xffffffffu, unusual3 != 0u);
+    if (any != 0u) {  // several periodic images can matter: the general routine
+        const Vec3 p1{shfl_d(pa, g), shfl_d(pa, g + 1), shfl_d(pa, g + 2)};
+        const Vec3 p2{shfl_d(pb, g), shfl_d(pb, g + 1), shfl_d(pb, g + 2)};
+        const Vec3 dir{shfl_d(u, 0), shfl_d(u, 1), shfl_d(u, 2)};
+        if (unusual3 != 0u) res = sweep_contact_general(p1, r1, p2, r2, dir, dist, L);
+    }
+    return touch ? 0.0 : res;
+}
+
+// The picked slot's record, spread over the warp: lane f holds field f of
+// the FP64 table (f < 21), and lane k entry k of RecInt. Each lane keeps its
+// own row's address (sm.rec_ptr), so that a record is one load instruction
+// per table: chosen among the tables by lane at each use, the loads went out
+// one after another (4400 cycles a record instead of about 600).
+enum RecInt : int { REC_N, REC_OFF, REC_CELL, REC_POS, REC_FINE, REC_PREV, REC_NEXT, REC_F4, REC_INTS = REC_F4 + 4 };
+struct WarpRec {
+    double f;
+    int i;
+};
+struct RecRows {
+    const double *f;
+    const int *i;
+    int shift;  // entry stride of the integer row, as a shift
+};
+template <class LS>
+__device__ __forceinline__ RecRows record_rows(const LS &sm, int lane) {
+    const DevBox &b = sm.R.box;
+    return RecRows{b.agg + size_t(lane < AGG_NFIELDS ? lane : 0) * size_t(b.nslots),
+                   lane < REC_INTS ? sm.rec_ptr[lane] : nullptr, lane >= REC_F4 ? 2 : 0};
+}
+__device__ __forceinline__ WarpRec load_record(const RecRows &rows, int slot) {
+    WarpRec r;
+    r.f = rows.f[slot];
+    r.i = rows.i != nullptr ? rows.i[size_t(slot) << rows.shift] : -1;
+    return r;
+}
+// The rows' addresses (all threads, once a launch; null: no such table).
+template <class LS>
+__device__ inline void record_rows_init(LS &sm) {
+    const DevBox &b = sm.R.box;
+    if (threadIdx.x != 0) return;
+    const bool fine = b.fine_div > 0;
+    sm.rec_ptr[REC_N] = b.agg_n;
+    sm.rec_ptr[REC_OFF] = b.agg_off;
+    sm.rec_ptr[REC_CELL] = b.agg_cell;
+    sm.rec_ptr[REC_POS] = b.cell_pos;
+    sm.rec_ptr[REC_FINE] = fine ? b.fine_cell : nullptr;
+    sm.rec_ptr[REC_PREV] = fine ? b.fine_prev : nullptr;
+    sm.rec_ptr[REC_NEXT] = fine ? b.fine_next : nullptr;
+    for (int k = 0; k < 4; ++k) sm.rec_ptr[REC_F4 + k] = reinterpret_cast<const int *>(b.agg_f4) + k;
+}
+
+// The contact query of the picked slot by warp 0. 'dl' is the direction's
+// component on lanes 0-2. Returns false when the block has to run it (long
+// lists or many pairs); then nothing was changed. Otherwise the answer and
+// the work counts are in 'o'.
+struct WarpAnswer {
+    double distance;
+    int ms, os, oslot, status;
+    int scanned, cells, cands, cand_spheres, refined;
+    unsigned t_scan;  // clock after the neighbourhood and the filter
+};
+template <class LS>
+__device__ __forceinline__ bool warp_query(const DevBox &b, LS &sm, int src, const WarpRec &rec, double dl, double full,
+                                           WarpAnswer &o) {
+    const DevScalars *sc = &sm.sc;
+    auto &W = sm.u.w;
+    const int lane = threadIdx.x & 31;
+    const unsigned all = 0xffffffffu;
+    // FP32 forms of the direction (lanes 0-2), the length and the largest
+    // r_max: one conversion for all of them
+    const float cf = float(lane == 3 ? full : (lane == 4 ? sc->maxradius : dl));
+    Sweep32 w;
+    w.px = __int_as_float(shfl_i(rec.i, REC_F4));
+    w.py = __int_as_float(shfl_i(rec.i, REC_F4 + 1));
+    w.pz = __int_as_float(shfl_i(rec.i, REC_F4 + 2));
+    const float rmax_f = __int_as_float(shfl_i(rec.i, REC_F4 + 3));
+    w.ux = shfl_f(cf, 0);
+    w.uy = shfl_f(cf, 1);
+    w.uz = shfl_f(cf, 2);
+    w.dist = shfl_f(cf, 3);
+    w.cx = 0.5f * w.dist * w.ux;
+    w.cy = 0.5f * w.dist * w.uy;
+    w.cz = 0.5f * w.dist * w.uz;
+    w.L = b.Lf;
+    w.invL = b.inv_Lf;
+    const float margin = b.margin_f + 1e-6f * w.dist;
+    w.zmax = fmaxf(fabsf(w.dist * w.ux), fmaxf(fabsf(w.dist * w.uy), fabsf(w.dist * w.uz)));
+    w.margin = margin;
+    const float reach_f = rmax_f + shfl_f(cf, 4);
+    // the Verlet and fine cell ranges, one axis on each of lanes 0-2
+    int lo = 0, n_c = 0, flo = 0, fn = 0;
+    const double x_ax = shfl_d(rec.f, AGG_X + (lane < 3 ? lane : 0));
+    const double rmax = shfl_d(rec.f, AGG_RMAX);
+    if (lane < 3) {
+        const float pf = lane == 0 ? w.px : (lane == 1 ? w.py : w.pz);
+        const float vf = w.dist * cf;
+        int hi = 0;
+        if (!neighborhood_axis_f32(pf, vf, reach_f, b.n_div, b.step_f, &lo, &hi))
+            neighborhood_axis_call(x_ax, full * dl, rmax + sc->maxradius, b.n_div, b.L, b.inv_L, &lo, &hi);
+        n_c = hi - lo + 1;
+        if (b.fine_div > 0) {  // widened as in block_query
+            const float flof = floorf((pf - reach_f + fminf(vf, 0.f)) * b.fine_step_f - 2e-3f);
+            const float fhif = floorf((pf + reach_f + fmaxf(vf, 0.f)) * b.fine_step_f + 2e-3f);
+            const bool part = (fhif - flof + 1.f < float(b.fine_div)) && flof > -1e6f && fhif < 1e6f;
+            flo = part ? int(flof) : 0;
+            fn = part ? int(fhif - flof + 1.f) : b.fine_div;
+        }
+    }
+    const int nd = b.n_div;
+    const int rlo0 = shfl_i(lo, 0), rlo1 = shfl_i(lo, 1), rlo2 = shfl_i(lo, 2);
+    const int nx = shfl_i(n_c, 0), ny = shfl_i(n_c, 1), nz = shfl_i(n_c, 2);
+    const bool live = sm.live.on != 0;
+    bool fine = false;
+    int n_scan = nx * ny * nz;
+    int total = 0;  // entries in the list
+    const int *list = W.queue;
+    if (live) {
+        list = sm.live.slot;
+        total = sm.live.n;
+        o.cells = 0;
+    } else {
+        int fn0 = 0, fn1 = 0, fn2 = 0, n_fine = 0;
+        if (b.fine_div > 0) {
+            fn0 = shfl_i(fn, 0);
+            fn1 = shfl_i(fn, 1);
+            fn2 = shfl_i(fn, 2);
+            n_fine = fn0 * fn1 * fn2;
+            const float alive = float(sc->n_alive);
+            const float cost_fine = float(n_fine) * (1.f + alive * b.inv_fine_cells);
+            const float cost_coarse = float(n_scan) * (1.f + alive * b.inv_cells);
+            fine = n_fine <= kFineMaxCells && cost_fine < cost_coarse;
+        }
+        const int n_cells = fine ? n_fine : n_scan;
+        if (n_cells > kWarpCells) return false;
+        o.cells = n_cells;
+        const int dy = fine ? fn1 : ny, dz = fine ? fn2 : nz, nf = fine ? b.fine_div : nd;
+        const int l0 = fine ? shfl_i(flo, 0) : rlo0, l1 = fine ? shfl_i(flo, 1) : rlo1, l2 = fine ? shfl_i(flo, 2) : rlo2;
+        // g -> (a, bb, c) by FP32 reciprocals, exact for these sizes
+        const int dyz = dy * dz;
+        const float inv_yz = 1.f / float(dyz), inv_z = 1.f / float(dz);
+        const int *heads = fine ? b.fine_head : b.cell_n;
+        int lin[kWarpCells / 32], h[kWarpCells / 32];
+#pragma unroll
+        for (int u = 0; u < kWarpCells / 32; ++u) {
+            const int g = u * 32 + lane;
+            h[u] = fine ? -1 : 0;
+            lin[u] = 0;
+            if (g < n_cells) {
+                const int a = int((float(g) + 0.5f) * inv_yz), r = g - a * dyz;
+                const int bb = int((float(r) + 0.5f) * inv_z), c = r - bb * dz;
+                lin[u] = (wrap_cell(l0 + a, nf) * nf + wrap_cell(l1 + bb, nf)) * nf + wrap_cell(l2 + c, nf);
+                h[u] = heads[lin[u]];
+            }
+        }
+        if (fine) {
+#pragma unroll
+            for (int u = 0; u < kWarpCells / 32; ++u) {
+                const unsigned m = __ballot_sync(all, h[u] >= 0);
+                if (h[u] >= 0) W.queue[total + __popc(m & lanes_below(lane))] = h[u];
+                total += __popc(m);
+            }
+        } else {
+            int cnt = 0;
+#pragma unroll
+            for (int u = 0; u < kWarpCells / 32; ++u) cnt += h[u];
+            int incl = cnt;
+#pragma unroll
+            for (int s = 1; s < 32; s <<= 1) {
+                const int y = __shfl_up_sync(all, incl, s);
+                if (lane >= s) incl += y;
+            }
+            total = shfl_i(incl, 31);
+            if (total > kWarpQueue) return false;
+            int at = incl - cnt;
+#pragma unroll
+            for (int u = 0; u < kWarpCells / 32; ++u) {
+                const int *items = b.cell_items + size_t(lin[u]) * b.cell_cap;
+#pragma unroll 1
+                for (int k = 0; k < h[u]; ++k) W.queue[at + k] = items[k];
+                at += h[u];
+            }
+        }
+        __syncwarp();
+    }
+    // the listed aggregates: those in the reference's neighbourhood that pass
+    // the FP32 screen wait for the FP64 filter, with their scan keys
+    bool found = false;
+    int n_screen = 0;
+    for (int k0 = 0, cnt = 0; k0 < total; k0 += cnt) {
+        cnt = min(32, total - k0);
+        const int slot = lane < cnt ? list[k0 + lane] : -1;
+        int nxt = -1, key = 0;
+        float4 of = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (slot >= 0) {
+            if (fine) nxt = b.fine_next[slot];
+            key = b.agg_cell[slot];
+            of = b.agg_f4[slot];
+        }
+        const int oa = wrap_cell((key & 1023) - rlo0, nd);
+        const int ob = wrap_cell(((key >> 10) & 1023) - rlo1, nd);
+        const int oc = wrap_cell((key >> 20) - rlo2, nd);
+        const bool in = slot >= 0 && oa < nx && ob < ny && oc < nz;
+        // the fine walk and the cells always hold the source; the live list
+        // counts it when its cell is in the neighbourhood
+        found = found || (slot == src && (!live || in));
+        const bool pass = in && slot != src && capsule_hit(w, of.x, of.y, of.z, rmax_f + of.w + margin);
+        const unsigned m = __ballot_sync(all, pass);
+        if (n_screen + __popc(m) > kWarpCands) return false;
+        if (pass) {
+            const int at = n_screen + __popc(m & lanes_below(lane));
+            W.scr_slot[at] = slot;
+            W.scr_key[at] = (long long)((oa * ny + ob) * nz + oc) * b.nslots + slot;
+        }
+        n_screen += __popc(m);
+        if (fine) {
+            const unsigned mn = __ballot_sync(all, nxt >= 0);
+            if (total + __popc(mn) > kWarpQueue) return false;
+            if (nxt >= 0) W.queue[total + __popc(mn & lanes_below(lane))] = nxt;
+            total += __popc(mn);
+        }
+        __syncwarp();
+    }
+    o.scanned = total;
+    o.status = ST_OK;
+    o.distance = CUDART_INF;
+    o.ms = o.os = o.oslot = -1;
+    o.cands = o.cand_spheres = o.refined = 0;
+    if (!__any_sync(all, found)) {
+        o.status = ST_VERLET;  // "Aggregate not on the verlet list"
+        o.t_scan = clock_lo();
+        return true;
+    }
+    // the exact bounding-sphere filter, ten neighbours at a time
+    const int gi = lane / 3, ax = lane - 3 * gi, g = 3 * gi;
+    const double x_g = shfl_d(rec.f, AGG_X + ax);
+    int nc = 0;
+    for (int k0 = 0; k0 < n_screen; k0 += 10) {
+        const bool act = lane < 30 && k0 + gi < n_screen;
+        const int slot = act ? W.scr_slot[k0 + gi] : src;
+        const double pb = A(b, AGG_X + ax, slot), r2 = A(b, AGG_RMAX, slot);
+        const double db = warp_sweep(g, ax, x_g, pb, rmax, r2, dl, full, b.L);
+        const bool pass = act && ax == 0 && dkey(db) < dkey(full);
+        const unsigned m = __ballot_sync(all, pass);
+        if (pass) {
+            const int at = nc + __popc(m & lanes_below(lane));
+            W.c_db[at] = dkey(db);
+            W.c_key[at] = W.scr_key[k0 + gi];
+            W.c_slot[at] = slot;
+        }
+        nc += __popc(m);
+    }
+    __syncwarp();
+    o.cands = nc;
+    o.t_scan = clock_lo();
+    if (nc == 0) return true;
+    // candidates in the order (d_b, scan key), with their spheres' prefix
+    const unsigned long long my_db = lane < nc ? W.c_db[lane] : ~0ULL;
+    const long long my_key = lane < nc ? W.c_key[lane] : 0;
+    const int my_slot = lane < nc ? W.c_slot[lane] : src;
+    const int my_n = b.agg_n[my_slot], my_off = b.agg_off[my_slot];
+    int rank = lane;
+    if (nc > 1) {
+        rank = 0;
+        for (int m = 0; m < nc; ++m) {
+            const unsigned long long dm = W.c_db[m];
+            rank += dm < my_db || (dm == my_db && W.c_key[m] < my_key);
+        }
+    }
+    __syncwarp();
+    if (lane < nc) {
+        W.s_db[rank] = my_db;
+        W.s_slot[rank] = my_slot;
+        W.s_off[rank] = my_off;
+        W.s_pre[rank] = my_n;
+    }
+    __syncwarp();
+    int n_other = 0;
+    {
+        const int cnt = lane < nc ? W.s_pre[lane] : 0;
+        int incl = cnt;
+        if (nc > 1) {
+#pragma unroll
+            for (int s = 1; s < 32; s <<= 1) {
+                const int y = __shfl_up_sync(all, incl, s);
+                if (lane >= s) incl += y;
+            }
+        }
+        n_other = shfl_i(incl, nc - 1);
+        __syncwarp();
+        if (lane < nc) W.s_pre[lane] = incl - cnt;
+    }
+    __syncwarp();
+    const int n_mov = shfl_i(rec.i, REC_N), off_m = shfl_i(rec.i, REC_OFF);
+    // pairs for the block: its screens and tiles pay off for more
+    if (n_mov > kWarpPairs || n_other > kWarpPairs || n_mov * n_other > kWarpPairs) return false;
+    o.cand_spheres = n_other;
+    const int *pool_id = sc->pool_sel ? b.pool_id[1] : b.pool_id[0];
+    const float4 *pool_pos = sc->pool_sel ? b.pool_pos[1] : b.pool_pos[0];
+    const int n_pairs = n_mov * n_other;
+    const float inv_mov = 1.f / float(n_mov);
+    int n_hit = 0;
+    for (int p0 = 0; p0 < n_pairs; p0 += 32) {
+        const int p = p0 + lane;
+        bool hit = false;
+        int r = 0, i = 0, jl = 0, pj = 0;
+        if (p < n_pairs) {
+            const int f = int((float(p) + 0.5f) * inv_mov);
+            i = p - f * n_mov;
+            while (r + 1 < nc && W.s_pre[r + 1] <= f) ++r;
+            jl = f - W.s_pre[r];
+            pj = W.s_off[r] + jl;
+            const float4 q = pool_pos[pj], pm = pool_pos[off_m + i];
+            Sweep32 wi = w;
+            wi.px = pm.x;
+            wi.py = pm.y;
+            wi.pz = pm.z;
+            hit = capsule_hit(wi, q.x, q.y, q.z, pm.w + q.w + margin);
+        }
+        const unsigned m = __ballot_sync(all, hit);
+        if (n_hit + __popc(m) > kWarpCands) return false;
+        if (hit) {
+            const int at = n_hit + __popc(m & lanes_below(lane));
+            W.p_r[at] = r;
+            W.p_ij[at] = (static_cast<unsigned long long>(i) << 32) | static_cast<unsigned>(jl);
+            W.p_si[at] = pool_id[off_m + i];
+            W.p_sj[at] = pool_id[pj];
+        }
+        n_hit += __popc(m);
+    }
+    __syncwarp();
+    o.refined = n_hit;
+    if (n_hit == 0) return true;
+    for (int k0 = 0; k0 < n_hit; k0 += 10) {
+        const bool act = lane < 30 && k0 + gi < n_hit;
+        const int k = act ? k0 + gi : 0;
+        const int si = W.p_si[k], sj = W.p_sj[k];
+        const double res = warp_sweep(g, ax, S(b, SPH_X + ax, si), S(b, SPH_X + ax, sj), S(b, SPH_R, si),
+                                      S(b, SPH_R, sj), dl, full, b.L);
+        if (act && ax == 0) W.p_key[k] = res < CUDART_INF ? dkey(res) : ~0ULL;
+    }
+    __syncwarp();
+    // the reference's ordered walk with early exits
+    const unsigned long long my_res = lane < n_hit ? W.p_key[lane] : ~0ULL;
+    const int my_r = lane < n_hit ? W.p_r[lane] : -1;
+    unsigned long long best = dkey(CUDART_INF);
+    int best_r = -1;
+    for (int r = 0; r < nc; ++r) {
+        if (best_r >= 0 && (best <= dkey(0.0) || best < W.s_db[r])) break;
+        unsigned long long v = my_r == r ? my_res : ~0ULL;
+        const unsigned m = __ballot_sync(all, v != ~0ULL);
+        if (m == 0u) continue;  // no finite pair: +inf never wins
+        if ((m & (m - 1u)) == 0u) {
+            v = __shfl_sync(all, v, __ffs(m) - 1);
+        } else {
+#pragma unroll
+            for (int s = 16; s > 0; s >>= 1) {
+                const unsigned long long y = __shfl_xor_sync(all, v, s);
+                v = y < v ? y : v;
+            }
+        }
+        if (v < best) {
+            best = v;
+            best_r = r;
+        }
+    }
+    if (best_r < 0) return true;
+    // among the candidate's equal minima the first (moving, other) pair
+    unsigned long long ij = my_r == best_r && my_res == best ? W.p_ij[lane] : ~0ULL;
+    unsigned m = __ballot_sync(all, ij != ~0ULL);
+    if ((m & (m - 1u)) != 0u) {
+        unsigned long long v = ij;
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) {
+            const unsigned long long y = __shfl_xor_sync(all, v, s);
+            v = y < v ? y : v;
+        }
+        m = __ballot_sync(all, ij == v);
+    }
+    const int win = __ffs(m) - 1;
+    o.distance = dkey_inv(best);
+    o.ms = W.p_si[win];
+    o.os = W.p_sj[win];
+    o.oslot = W.s_slot[best_r];
+    return true;
+}
+
+// A slot's place after a move: the new centre (lanes 0-2 an axis each) and
+// its cells.
+struct WarpPlace {
+    double x;
+    float xf;
+    int key, fcell;
+};
+__device__ __forceinline__ WarpPlace warp_place(const DevBox &b, double x0, double dl, double move) {
+    const int lane = threadIdx.x & 31;
+    WarpPlace p;
+    int vc = 0, fc = 0;
+    p.x = 0.0;
+    p.xf = 0.f;
+    if (lane < 3) {
+        p.x = wrap_position(x0 + dl * move, b.L);
+        p.xf = float(p.x);
+        vc = verlet_coord_dev(b, p.x, p.xf);
+        if (b.fine_div > 0) fc = fine_index_near(p.xf, b.fine_step_f, b.fine_div);
+    }
+    p.key = cell_key(shfl_i(vc, 0), shfl_i(vc, 1), shfl_i(vc, 2));
+    const int nf = b.fine_div;
+    p.fcell = nf > 0 ? (shfl_i(fc, 0) * nf + shfl_i(fc, 1)) * nf + shfl_i(fc, 2) : -1;
+    return p;
+}
+
+// Aggregate::translate (aggregat.cpp:148-161) of the picked slot's fields and
+// members by warp 0 (as block_translate), without the grids. The members'
+// first ten (sid, rel: member lane / 3, axis lane % 3) are already loaded.
+__device__ __forceinline__ void warp_translate(const DevBox &b, int pool_sel, int slot, const WarpRec &rec,
+                                               const WarpPlace &to, int sid, double rel) {
+    const int lane = threadIdx.x & 31;
+    const int gi = lane / 3, ax = lane - 3 * gi;
+    const int n = shfl_i(rec.i, REC_N), off = shfl_i(rec.i, REC_OFF);
+    const double r0 = shfl_d(rec.f, AGG_RX + (lane < 3 ? lane : 0));
+    if (lane < 3) {
+        A(b, AGG_X + lane, slot) = to.x;
+        reinterpret_cast<float *>(b.agg_f4 + slot)[lane] = to.xf;
+    }
+    const double ref_ax = shfl_d(to.x - r0, ax);
+    const int *pool_id = pool_sel ? b.pool_id[1] : b.pool_id[0];
+    float *pf = reinterpret_cast<float *>((pool_sel ? b.pool_pos[1] : b.pool_pos[0]) + off);
+    if (sid >= 0) {
+        const double v = ref_ax + rel;
+        S(b, SPH_X + ax, sid) = v;
+        pf[4 * gi + ax] = float(v);  // the entry's radius stays as it is
+    }
+#pragma unroll 1
+    for (int k0 = 10; k0 < n; k0 += 40) {
+        int s[4];
+        double rl[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int k = k0 + 10 * u + gi;
+            s[u] = lane < 30 && k < n ? pool_id[off + k] : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) rl[u] = s[u] >= 0 ? S(b, SPH_RX + ax, s[u]) : 0.0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (s[u] >= 0) {
+                const double v = ref_ax + rl[u];
+                S(b, SPH_X + ax, s[u]) = v;
+                pf[4 * (k0 + 10 * u + gi) + ax] = float(v);
+            }
+    }
+}
+
+// What regrid_to reads to move the slot to 'to', loaded ahead: in 'a' lane 0
+// has the length of the new Verlet cell's list, lane 1 that of the old one's,
+// lane 2 the head of the new fine cell's (a second round of loads then
+// depends on it: warp_regrid_items).
+struct WarpGrid {
+    int a, b;
+};
+__device__ __forceinline__ int warp_regrid_heads(const DevBox &b, const WarpRec &rec, const WarpPlace &to) {
+    const int lane = threadIdx.x & 31;
+    const int old_key = shfl_i(rec.i, REC_CELL);
+    if (lane == 2 && b.fine_div > 0) return b.fine_head[to.fcell];
+    return lane < 2 ? b.cell_n[cell_index(b, lane == 0 ? to.key : old_key)] : -1;
+}
+// Lane 0: the old cell's last item, lane 1: its item at the slot's place.
+__device__ __forceinline__ int warp_regrid_items(const DevBox &b, const WarpRec &rec, int heads) {
+    const int lane = threadIdx.x & 31;
+    const int n_old = shfl_i(heads, 1), pos = shfl_i(rec.i, REC_POS), old_key = shfl_i(rec.i, REC_CELL);
+    const int k = lane == 0 ? n_old - 1 : pos;
+    return lane < 2 && k >= 0 && k < n_old ? b.cell_items[size_t(cell_index(b, old_key)) * b.cell_cap + k] : -1;
+}
+// regrid_to from those loads (lane 0 stores).
+__device__ __forceinline__ void warp_regrid(const DevBox &b, int slot, const WarpRec &rec, const WarpPlace &to,
+                                            const WarpGrid &g) {
+    const int lane = threadIdx.x & 31;
+    const int old_key = shfl_i(rec.i, REC_CELL), pos = shfl_i(rec.i, REC_POS);
+    const int fold = shfl_i(rec.i, REC_FINE), fprev = shfl_i(rec.i, REC_PREV), fnext = shfl_i(rec.i, REC_NEXT);
+    const int n_new = shfl_i(g.a, 0), n_old = shfl_i(g.a, 1), fhead = shfl_i(g.a, 2);
+    const int last = shfl_i(g.b, 0), item = shfl_i(g.b, 1);
+    if (to.key != old_key && (item != slot || n_new >= b.cell_cap)) {
+        // not where recorded, or a full cell: the general form
+        if (lane == 0) regrid_to(b, slot, to.key, to.fcell);
+        return;
+    }
+    if (lane == 0) {
+        if (to.key != old_key) {
+            const int c = cell_index(b, to.key), old = cell_index(b, old_key);
+            b.cell_items[size_t(old) * b.cell_cap + pos] = last;
+            b.cell_pos[last] = pos;
+            b.cell_n[old] = n_old - 1;
+            b.cell_items[size_t(c) * b.cell_cap + n_new] = slot;
+            b.cell_pos[slot] = n_new;
+            b.cell_n[c] = n_new + 1;
+            b.agg_cell[slot] = to.key;
+        }
+        if (to.fcell != fold) {
+            if (fold >= 0) {
+                if (fprev >= 0) b.fine_next[fprev] = fnext; else b.fine_head[fold] = fnext;
+                if (fnext >= 0) b.fine_prev[fnext] = fprev;
+            }
+            b.fine_next[slot] = fhead;
+            b.fine_prev[slot] = -1;
+            if (fhead >= 0) b.fine_prev[fhead] = slot;
+            b.fine_head[to.fcell] = slot;
+            b.fine_cell[slot] = to.fcell;
+        }
+    }
+}
+
+// The merge of the step's contact by warp 0: block_merge (with no volume and
+// surface correction), the physics and the pick tree of commit_merge, one
+// sphere of the merged aggregate per lane. The FP64 chains are cut by doing
+// what is independent on different lanes of one instruction: the seven
+// ordered sums and the overlap's, the five quotients at the end, the two
+// reciprocals after the physics; a tree update adds differences to the
+// ancestors (the weights are integers, so the sums are the same) instead of
+// reading 32 children a level. Returns WM_BLOCK when the block has to do it
+// (more than 32 spheres, or the member pool is full; nothing was changed).
+enum WarpMergeResult : int { WM_BLOCK, WM_DONE, WM_TREE, WM_LIVE };
+template <class LS>
+__device__ __noinline__ int warp_merge() {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    LS &sm = *reinterpret_cast<LS *>(smem_raw);
+    const BoxRun &R = sm.R;
+    const DevBox &b = R.box;
+    DevScalars *sc = &sm.sc;
+    RunState &st = sm.st;
+    auto &M = sm.u.wm;
+    const unsigned all = 0xffffffffu;
+    const int lane = threadIdx.x & 31, a3 = lane < 3 ? lane : 0;
+    const int ms = sm.ms, os = sm.os, mslot = sm.mslot, cslot = sm.cslot;
+    const int keep = min(mslot, cslot), removed = max(mslot, cslot);
+    const int my = mslot == keep ? ms : os, oth = mslot == keep ? os : ms;
+    // round 1: both records, the two spheres, the leaves
+    const RecRows rows = record_rows(sm, lane);
+    const WarpRec rk = load_record(rows, keep), rr = load_record(rows, removed);
+    const double pm = S(b, SPH_X + a3, ms), po = S(b, SPH_X + a3, os);
+    const double rms = S(b, SPH_R, ms), ros = S(b, SPH_R, os);
+    const double rel_my = S(b, SPH_RX + a3, my), rel_oth = S(b, SPH_RX + a3, oth);
+    const unsigned long long w_keep = R.tree[R.tree_off[0] + keep], w_removed = R.tree[R.tree_off[0] + removed];
+    const int nk = shfl_i(rk.i, REC_N), nr = shfl_i(rr.i, REC_N), n = nk + nr;
+    const int off_keep = shfl_i(rk.i, REC_OFF), off_rem = shfl_i(rr.i, REC_OFF);
+    const int new_off = sc->pool_top;
+    if (n > 32 || keep == removed || new_off + n > b.pool_cap) return WM_BLOCK;
+    {
+        const double d = wrap_distance(pm - po, b.L);
+        const double d2 = sum3(d * d, 0);
+        const double s = rms + ros;
+        if (!(dkey(d2 - s * s) <= dkey(kContactEpsilon))) return WM_DONE;  // the spheres no longer touch
+    }
+    const double diff = (rel_my + wrap_distance(my == ms ? po - pm : pm - po, b.L)) - rel_oth;
+    // round 2: the members, and the removed slot's cell
+    int *pool_id = sc->pool_sel ? b.pool_id[1] : b.pool_id[0];
+    float4 *pool_pos = sc->pool_sel ? b.pool_pos[1] : b.pool_pos[0];
+    const bool act = lane < n, gone = act && lane >= nk;
+    const int at = lane < nk ? off_keep + lane : off_rem + (lane - nk);
+    const int sid = act ? pool_id[at] : 0;
+    float4 pp = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (act) pp = pool_pos[at];
+    const int cell_r = cell_index(b, shfl_i(rr.i, REC_CELL)), pos_r = shfl_i(rr.i, REC_POS);
+    const int n_cell_r = b.cell_n[cell_r];
+    // round 3: the spheres
+    double r = 0.0, vol = 0.0, surf = 0.0, rx = 0.0, ry = 0.0, rz = 0.0;
+    if (act) {
+        r = S(b, SPH_R, sid);
+        vol = S(b, SPH_VOLUME, sid);
+        surf = S(b, SPH_SURFACE, sid);
+        rx = S(b, SPH_RX, sid);
+        ry = S(b, SPH_RY, sid);
+        rz = S(b, SPH_RZ, sid);
+    }
+    const double ref = S(b, SPH_X + a3, shfl_i(sid, 0));
+    int *items = b.cell_items + size_t(cell_r) * b.cell_cap;
+    const bool listed = pos_r >= 0 && pos_r < n_cell_r;
+    const int at_pos = listed ? items[pos_r] : -1, last = listed ? items[n_cell_r - 1] : -1;
+    {
+        const double dx = shfl_d(diff, 0), dy = shfl_d(diff, 1), dz = shfl_d(diff, 2);
+        const double fx = shfl_d(ref, 0), fy = shfl_d(ref, 1), fz = shfl_d(ref, 2);
+        if (gone) {  // relabel and shift the removed aggregate's spheres
+            rx = rx + dx;
+            ry = ry + dy;
+            rz = rz + dz;
+            const double x = rx + fx, y = ry + fy, z = rz + fz;
+            b.sph_slot[sid] = keep;
+            S(b, SPH_RX, sid) = rx;
+            S(b, SPH_RY, sid) = ry;
+            S(b, SPH_RZ, sid) = rz;
+            S(b, SPH_X, sid) = x;
+            S(b, SPH_Y, sid) = y;
+            S(b, SPH_Z, sid) = z;
+            pp.x = float(x);
+            pp.y = float(y);
+            pp.z = float(z);
+        }
+    }
+    if (act) {
+        pool_id[new_off + lane] = sid;
+        pool_pos[new_off + lane] = pp;
+        b.sph_volw[sid] = vol;
+        M.rel[0][lane] = rx;
+        M.rel[1][lane] = ry;
+        M.rel[2][lane] = rz;
+        M.term[0][lane] = vol;
+        M.term[1][lane] = surf;
+        M.term[2][lane] = rx * vol;
+        M.term[3][lane] = ry * vol;
+        M.term[4][lane] = rz * vol;
+        M.term[5][lane] = vol * (r * r);
+        M.term[6][lane] = r;
+    }
+    if (lane == 0) {
+        b.agg_off[keep] = new_off;
+        b.agg_n[keep] = n;
+        b.agg_n[removed] = 0;
+        sc->pool_top = new_off + n;
+        sc->n_alive -= 1;
+    }
+    // the removed slot leaves the grids
+    const int prev_r = shfl_i(rr.i, REC_PREV), next_r = shfl_i(rr.i, REC_NEXT), fine_r = shfl_i(rr.i, REC_FINE);
+    if (lane == 0) {
+        if (at_pos == removed) {
+            items[pos_r] = last;
+            b.cell_pos[last] = pos_r;
+            b.cell_pos[removed] = -1;
+            b.cell_n[cell_r] = n_cell_r - 1;
+        } else {
+            cell_remove(b, cell_r, removed);
+        }
+        if (fine_r >= 0) {
+            if (prev_r >= 0) b.fine_next[prev_r] = next_r; else b.fine_head[fine_r] = next_r;
+            if (next_r >= 0) b.fine_prev[next_r] = prev_r;
+            b.fine_cell[removed] = -1;
+        }
+    }
+    __syncwarp();
+    // contact pairs i < j in (i, j) order: an FP32 screen with the margins of
+    // block_pair_scan, then the exact test
+    int P = 1;
+    if (n == 2) {
+        if (lane == 0) M.pair[0] = 1;  // i = 0, j = 1
+    } else {
+        const float fx = float(rx), fy = float(ry), fz = float(rz), fr = pp.w;
+        const float ext = act ? fabsf(fx) + fabsf(fy) + fabsf(fz) + fr : 0.f;
+        const float margin = 1.0e-5f * __int_as_float(__reduce_max_sync(all, __float_as_int(ext)));
+        P = 0;
+        for (int i = 0; i + 1 < n; ++i) {
+            const float dx = shfl_f(fx, i) - fx, dy = shfl_f(fy, i) - fy, dz = shfl_f(fz, i) - fz;
+            const float reach = (shfl_f(fr, i) + fr) * 1.0001f + margin;
+            const bool hit = act && lane > i && __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz)) <= reach * reach;
+            const unsigned m = __ballot_sync(all, hit);
+            if (hit) M.pair[P + __popc(m & lanes_below(lane))] = static_cast<unsigned short>((i << 8) | lane);
+            P += __popc(m);
+        }
+    }
+    __syncwarp();
+    int Pc = 0;
+    for (int p0 = 0; p0 < P; p0 += 32) {
+        const bool has = p0 + lane < P;
+        const int ij = has ? M.pair[p0 + lane] : 1;
+        const int i = ij >> 8, j = ij & 255;
+        const double ex = M.rel[0][i] - M.rel[0][j], ey = M.rel[1][i] - M.rel[1][j], ez = M.rel[2][i] - M.rel[2][j];
+        const double dist = fp64_sqrt(ex * ex + ey * ey + ez * ez);
+        const double rsum = M.term[6][i] + M.term[6][j];
+        const bool pass = has && nonneg_le(dist, (1. + kCoordinationEpsilon) * rsum);
+        const double term = 2.0 * fp64_div(rsum - dist, rsum);
+        const unsigned m = __ballot_sync(all, pass);
+        if (pass) M.ov[Pc + __popc(m & lanes_below(lane))] = term;
+        Pc += __popc(m);
+    }
+    __syncwarp();
+    // the ordered sums: the seven series on lanes 0-6, the overlap's on lane 7
+    double acc = 0.0;
+    {
+        const double *v = lane < 7 ? M.term[lane] : M.ov;
+        const int lim = lane < 7 ? n : (lane == 7 ? Pc : 0), most = max(n, Pc);
+#pragma unroll 4
+        for (int k = 0; k < most; ++k) acc = acc + (k < lim ? v[k] : 0.0);
+    }
+    const double V = shfl_d(acc, 0), Sf = shfl_d(acc, 1);
+    if (dbits(V) <= 0 || dbits(Sf) <= 0) {
+        if (lane == 0) {
+            sc->status = ST_VOL_SURF;
+            st.status = ST_VOL_SURF;
+            sm.stop = 1;
+        }
+        __syncwarp();
+        return WM_DONE;
+    }
+    const double cm = fp64_div(acc, V);  // lanes 2-4: the centre of mass
+    const double cx = shfl_d(cm, 2), cy = shfl_d(cm, 3), cz = shfl_d(cm, 4);
+    const double dx = rx - cx, dy = ry - cy, dz = rz - cz;
+    const double dcen = fp64_sqrt(dx * dx + dy * dy + dz * dz);
+    long long rmax_bits = act ? dbits(r + dcen) : 0;  // non-negative: integer order
+    M.term[7][lane] = vol * (dcen * dcen);
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+        const long long y = __shfl_xor_sync(all, rmax_bits, s);
+        rmax_bits = y > rmax_bits ? y : rmax_bits;
+    }
+    const double rmax = __longlong_as_double(rmax_bits);
+    __syncwarp();
+    double arg = 0.0;
+#pragma unroll 4
+    for (int k = 0; k < n; ++k) arg = arg + M.term[7][k];
+    // the quotients of the fields, one per lane: Rg's, the mean diameter, the
+    // mean sphere volume, overlap and coordination
+    const double nd = double(n), pd = double(2 * Pc);
+    const double brg = shfl_d(acc, 5), sum_r = shfl_d(acc, 6), sum_ov = shfl_d(acc, 7);
+    const double prod = (lane == 0 ? 3. / 5. : 2.0) * (lane == 0 ? brg : sum_r);
+    const double num = lane == 0 ? arg + prod : (lane == 1 ? prod : (lane == 2 ? V : (lane == 3 ? sum_ov : pd)));
+    const double den = lane == 0 ? V : (lane == 3 ? pd : nd);
+    const double quo = fp64_div(num, den);
+    const double rg = fp64_sqrt(fabs(shfl_d(quo, 0)));
+    const double dp = shfl_d(quo, 1), vol_pp = shfl_d(quo, 2);
+    const double overlapping = Pc > 0 ? shfl_d(quo, 3) : 0.0, coordination = Pc > 0 ? shfl_d(quo, 4) : 0.0;
+    const double x = wrap_position(ref + shfl_d(cm, 2 + a3), b.L);  // lanes 0-2
+    const float cf = float(lane < 3 ? x : (lane == 3 ? rmax : (lane == 4 ? V : (lane == 5 ? vol_pp : half_of(dp)))));
+    const float4 ph = physics_f32(R.phys, shfl_f(cf, 6), shfl_f(cf, 4), shfl_f(cf, 5));
+    const double phd = double(lane == 0 ? ph.x : (lane == 1 ? ph.y : (lane == 2 ? ph.z : ph.w)));
+    // lane 0: Rg / (dp / 2), lane 2: 1 / time step
+    const double rec = fp64_div(lane == 0 ? rg : 1.0, lane == 0 ? half_of(dp) : phd);
+    unsigned long long wk = __double2ull_rn(fmin(rec * st.tree_scale, double(kTreeHeadroom)));
+    wk = __shfl_sync(all, wk > 0ULL ? wk : 1ULL, 2);
+    const double time = (shfl_d(rk.f, AGG_TIME) + shfl_d(rr.f, AGG_TIME)) - st.time;
+    if (lane < 3) {
+        A(b, AGG_X + lane, keep) = x;
+        reinterpret_cast<float *>(b.agg_f4 + keep)[lane] = cf;
+    }
+    if (lane >= 2 && lane < 5) A(b, AGG_RX + lane - 2, keep) = cm;
+    if (lane < 4) A(b, lane == 0 ? AGG_F_AGG : (lane == 1 ? AGG_D_M : (lane == 2 ? AGG_TIME_STEP : AGG_LPM)), keep) = phd;
+    if (lane == 3) reinterpret_cast<float *>(b.agg_f4 + keep)[3] = cf;
+    int vc = 0, fc = 0;
+    if (lane < 3) {
+        vc = verlet_coord_dev(b, x, cf);
+        if (b.fine_div > 0) fc = fine_index(cf, b.fine_step_f, b.fine_div);
+    }
+    const int nf = b.fine_div;
+    const int key = cell_key(shfl_i(vc, 0), shfl_i(vc, 1), shfl_i(vc, 2));
+    const int fcell = nf > 0 ? (shfl_i(fc, 0) * nf + shfl_i(fc, 1)) * nf + shfl_i(fc, 2) : -1;
+    const int cell_k = shfl_i(rk.i, REC_CELL), fine_k = shfl_i(rk.i, REC_FINE);
+    const unsigned long long total = st.tree_total - w_keep - w_removed + wk;
+    if (lane == 0) {
+        A(b, AGG_RG, keep) = rg;
+        A(b, AGG_RMAX, keep) = rmax;
+        A(b, AGG_VOLUME, keep) = V;
+        A(b, AGG_SURFACE, keep) = Sf;
+        A(b, AGG_DP, keep) = dp;
+        A(b, AGG_OVERLAPPING, keep) = overlapping;
+        A(b, AGG_COORDINATION_NUMBER, keep) = coordination;
+        A(b, AGG_DG_OVER_DP, keep) = rec;
+        A(b, AGG_TIME, keep) = time;
+        if (key != cell_k || fcell != fine_k) regrid_to(b, keep, key, fcell);
+        if (dbits(rmax) > dbits(sc->maxradius)) sc->maxradius = rmax;
+        sm.merged = 1;
+        st.c_merged_spheres += n;
+        st.c_merge_pairs += Pc;
+    }
+    // the pick tree, a level on each lane
+    if (lane < R.tree_levels) {
+        const int sh = 5 * lane, gk = keep >> sh, gr = removed >> sh, co = sm.tree.coff[lane];
+        unsigned long long *lev = R.tree + R.tree_off[lane];
+        unsigned long long *own = sm.tree.v + (co >= 0 ? co : 0);
+        unsigned long long vr = 0ULL, vk = wk;
+        if (lane > 0) {
+            vr = co >= 0 ? own[gr] : lev[gr];
+            vk = gk == gr ? vr : (co >= 0 ? own[gk] : lev[gk]);
+            vr -= w_removed;
+            vk = (gk == gr ? vr : vk) - w_keep + wk;
+        }
+        if (gk != gr) {
+            lev[gr] = vr;
+            if (co >= 0) own[gr] = vr;
+        }
+        lev[gk] = vk;
+        if (co >= 0) own[gk] = vk;
+    }
+    const bool rescale = total > kTreeHeadroom;  // a new scale keeps the total clear of 2^64
+    if (lane == 0) tree_total_to_state(st, total);
+    if (sm.live.on) warp_live_merge(sm.live, keep, removed, wk);
+    __syncwarp();
+    if (rescale) return WM_TREE;
+    return !sm.live.on && sm.live.allow && sc->n_alive <= sm.live.max ? WM_LIVE : WM_DONE;
+}
+
+// Warp 0: MC steps until the block is needed or the run ends (sm.left counts
+// the steps still allowed; t_phase is the clock at the start of the phase).
+// Returns the operation (StepOp). The counters are summed in registers and
+// added to the loop state every so often.
+template <class LS>
+__device__ __forceinline__ int warp_steps(LS &sm, int phase, unsigned &t_phase) {
+    const int lane = threadIdx.x & 31;
+    const BoxRun &R = sm.R;
+    const DevBox &b = R.box;
+    RunState &st = sm.st;
+    const int pool_sel = sm.sc.pool_sel;  // changes only in the block's operations
+    const int *pool_id = pool_sel ? b.pool_id[1] : b.pool_id[0];
+    const RecRows rows = record_rows(sm, lane);
+    const int gi = lane / 3, ax = lane - 3 * gi, a3 = lane < 3 ? lane : 0;
+    const bool growth = R.phys.growth != 0;
+    // members translated here; more are the block's (one warp does them all)
+    const int move_max = blockDim.x > 32 ? kWarpMove : INT_MAX;
+    bool finished = st.finished || st.status != ST_OK || sm.stop;
+    // steps until the counters are added to the loop state
+    int quota = 0, n_done = 0;
+    unsigned n_mov = 0, n_scanned = 0, n_cells = 0, cyc_pick = 0, cyc_query = 0, cyc_scan = 0, cyc_move = 0, cyc_end = 0;
+    int n_query = 0;
+    // the step under way
+    int slot = sm.slot, contact = sm.contact, status = ST_OK;
+    double full = sm.full, move = sm.move, dl = lane < 3 ? sm.dir[lane] : 0.0;
+    WarpRec rec{0.0, -1};
+    bool have = false;  // the record is loaded
+    auto flush = [&]() {
+        if (lane == 0) {
+            sm.left -= n_done;
+            st.n_iter_without_event += n_done;
+            st.steps += n_done;
+            st.c_queries += n_query;
+            st.c_mov += n_mov;
+            st.c_scanned += n_scanned;
+            st.c_cells += n_cells;
+            st.cyc_pick += cyc_pick;
+            st.cyc_query += cyc_query;
+            st.cyc_qscan += cyc_scan;
+            if (n_query > 0) st.cyc_qpairs += (long long)cyc_query - (long long)cyc_scan;
+            st.cyc_move += cyc_move;
+            st.cyc_merge += cyc_end;
+        }
+        __syncwarp();
+        n_done = n_query = 0;
+        n_mov = n_scanned = n_cells = cyc_pick = cyc_query = cyc_scan = cyc_move = cyc_end = 0;
+    };
+    int op = STEP_EXIT;
+    for (;;) {
+        if (phase == PH_START) {
+            op = STEP_EXIT;
+            if (n_done >= quota) {
+                flush();
+                quota = int(min(sm.left, 256LL));
+            }
+            if (quota <= 0 || finished) break;
+            if (sm.deadline != 0ULL) {
+                // a time-capped launch: checked before every step, so that a
+                // box of expensive steps does not hold the launch past the cap
+                const int over = lane == 0 && global_ns() >= sm.deadline;
+                if (shfl_i(over, 0)) break;
+            }
+            t_phase = clock_lo();
+            // the step's three rand() values, one on each of lanes 0-2 (each
+            // needs values at least three places back)
+            int rnd = 0;
+            {
+                const int pos = st.rng.pos;
+                int k = pos + a3;
+                k -= k >= 34 ? 34 : 0;
+                const uint32_t v = st.rng.r[k >= 3 ? k - 3 : k + 31] + st.rng.r[k >= 31 ? k - 31 : k + 3];
+                __syncwarp();
+                if (lane < 3) st.rng.r[k] = v;
+                if (lane == 0) st.rng.pos = pos >= 31 ? pos - 31 : pos + 3;
+                rnd = int(v >> 1);
+                __syncwarp();
+            }
+            const unsigned long long r0 = static_cast<unsigned long long>(shfl_i(rnd, 0)), total = st.tree_total;
+            unsigned long long t = (__umul64hi(r0, total) << 33) | ((r0 * total) >> 31);
+            // the pick; the leaves' load is under way while the direction
+            // (direction_from, an axis on each of lanes 0-2) is formed
+            const bool live = sm.live.on != 0;
+            int base = 0;
+            unsigned long long leaf = 0ULL;
+            if (!live) {
+                int node = 0;
+#pragma unroll 1
+                for (int lev = R.tree_levels - 1; lev > 0; --lev)
+                    node = node * kTreeFan + tree_pick_child(tree_children(R, sm.tree, lev, node * kTreeFan), t);
+                base = node * kTreeFan;
+                leaf = tree_children(R, sm.tree, 0, base);
+            }
+            {
+                const float u1 = float(shfl_i(rnd, 1)) * (1.0f / 2147483647.0f);
+                const float u2 = float(shfl_i(rnd, 2)) * (1.0f / 2147483647.0f);
+                const float cpf = 1.f - 2.f * u2;
+                const float spf = 2.f * sqrtf(u2 * (1.f - u2));
+                float sth, cth;
+                sincospif(2.f * u1, &sth, &cth);
+                const double d = double(lane == 0 ? spf * cth : (lane == 1 ? spf * sth : cpf));
+                const double k = 1.5 - 0.5 * sum3(d * d, 0);
+                dl = d * k;
+            }
+            slot = live ? live_sample(sm.live, t) : base + tree_pick_child(leaf, t);
+            const bool ok = slot >= 0 && slot < b.nslots;
+            rec = load_record(rows, ok ? slot : 0);
+            const int n = shfl_i(rec.i, REC_N);
+            if (!ok || n == 0) {
+                status = ST_UNKNOWN;  // the tree lost a live slot: stop this box
+                break;
+            }
+            have = true;
+            contact = 0;
+            full = shfl_d(rec.f, AGG_LPM);
+            move = full;
+            const unsigned now = clock_lo();
+            cyc_pick += now - t_phase;
+            t_phase = now;
+            if (R.lim.with_collisions) {
+                WarpAnswer o;
+                if (!warp_query(b, sm, slot, rec, dl, full, o)) {
+                    op = STEP_QUERY;
+                    break;
+                }
+                n_query += 1;
+                n_mov += n;
+                n_scanned += o.scanned;
+                n_cells += o.cells;
+                if (o.cands > 0 && lane == 0) {
+                    st.c_candidates += o.cands;
+                    st.c_cand_spheres += o.cand_spheres;
+                    st.c_refined += o.refined;
+                }
+                if (o.status != ST_OK) {
+                    status = o.status;
+                    break;
+                }
+                if (dkey(o.distance) <= dkey(full)) {
+                    contact = 1;
+                    move = o.distance;
+                    if (lane == 0) {
+                        sm.ms = o.ms;
+                        sm.os = o.os;
+                        sm.oslot = o.oslot;
+                    }
+                }
+                const unsigned done = clock_lo();
+                cyc_scan += o.t_scan - t_phase;
+                cyc_query += done - t_phase;
+                t_phase = done;
+            }
+            phase = PH_QUERIED;
+        }
+        if (phase == PH_QUERIED) {
+            if (!have) {  // back from the block's query
+                if (finished) break;
+                rec = load_record(rows, slot);
+                have = true;
+                const unsigned now = clock_lo();
+                if (lane == 0) st.cyc_query += now - t_phase;
+                t_phase = now;
+            }
+            const int n = shfl_i(rec.i, REC_N), off = shfl_i(rec.i, REC_OFF);
+            if (n > move_max) {
+                op = STEP_MOVE;
+                break;
+            }
+            // the members' ids and the grids' heads, then what hangs on them,
+            // are loaded together
+            const int sid = lane < 30 && gi < n ? pool_id[off + gi] : -1;
+            const WarpPlace to = warp_place(b, shfl_d(rec.f, AGG_X + a3), dl, move);
+            const bool cell = to.key != shfl_i(rec.i, REC_CELL), regrid = cell || to.fcell != shfl_i(rec.i, REC_FINE);
+            WarpGrid grid{-1, -1};
+            if (regrid) grid.a = warp_regrid_heads(b, rec, to);
+            const double rel = sid >= 0 ? S(b, SPH_RX + ax, sid) : 0.0;
+            if (cell) grid.b = warp_regrid_items(b, rec, grid.a);
+            if (regrid) warp_regrid(b, slot, rec, to, grid);
+            warp_translate(b, pool_sel, slot, rec, to, sid, rel);
+            phase = PH_MOVED;
+        }
+        if (phase == PH_MOVED) {
+            // without contact the move is the full lpm and the ratio is 1; the
+            // aggregate's proper time and the box's advance together
+            if (!have && lane == AGG_TIME) rec.f = A(b, AGG_TIME, slot);
+            const double ratio = contact ? fp64_div(move, full) + 0.0 : 1.0;
+            const double dt = contact ? st.inv_weight * ratio : st.inv_weight;
+            const double then = (lane == AGG_TIME ? rec.f : st.time) + dt;
+            if (lane == AGG_TIME) A(b, AGG_TIME, slot) = then;
+            __syncwarp();
+            if (lane == 0) st.time = then;
+            const unsigned now = clock_lo();
+            cyc_move += now - t_phase;
+            t_phase = now;
+            if (contact || growth) {
+                const double own = have ? shfl_d(rec.f, AGG_TIME_STEP) : sm.dt_indiv;
+                if (lane == 0) {
+                    sm.slot = slot;
+                    sm.mslot = slot;
+                    sm.cslot = sm.oslot;
+                    sm.merged = 0;
+                    sm.try_merge = contact;
+                    sm.step_dt = dt;
+                    sm.step_dt_indiv = contact ? own * ratio : own;
+                }
+                __syncwarp();
+                if (growth) {
+                    op = STEP_REACT;
+                    break;
+                }
+                op = STEP_MERGE;
+                const int did = b.volsurf == VS_NONE ? warp_merge<LS>() : WM_BLOCK;
+                if (did == WM_BLOCK) break;
+                op = did == WM_TREE ? STEP_TREE : STEP_LIVE;
+                if (did != WM_DONE) break;
+                phase = PH_MERGED;
+            }
+        }
+        if (phase == PH_REACTED) {
+            if (finished) break;
+            if (sm.try_merge) {
+                op = STEP_MERGE;
+                break;
+            }
+            phase = PH_MERGED;
+        }
+        if (phase == PH_MERGED) {
+            op = STEP_EXIT;
+            if (finished || sm.stop) break;
+            if (growth) {
+                op = STEP_UPDATE;
+                break;
+            }
+            phase = PH_END;
+        }
+        // the end of the step
+        __syncwarp();
+        if (phase == PH_END) {  // after a contact or surface reactions
+            flush();
+            if (lane == 0) {
+                sm.left -= 1;
+                step_end(R, sm);
+            }
+            __syncwarp();
+            quota = 0;
+            finished = st.finished != 0;
+        } else {
+            n_done += 1;
+            const long long iter_limit = R.lim.n_iter_without_event_limit;
+            const double time_limit = R.lim.physical_time_limit;
+            finished = (iter_limit > 0 && st.n_iter_without_event + n_done >= iter_limit) ||
+                       (dbits(time_limit) > 0 && nonneg_le(time_limit, st.time));
+            if (finished && lane == 0) st.finished = 1;
+        }
+        const unsigned now = clock_lo();
+        cyc_end += now - t_phase;
+        t_phase = now;
+        have = false;
+        phase = PH_START;
+    }
+    // what the block's operation and the next entry need
+    flush();
+    if (lane < 3) sm.dir[lane] = dl;
+    if (have && lane == AGG_TIME_STEP) sm.dt_indiv = rec.f;
+    if (lane == 0) {
+        if (status != ST_OK) st.status = status;
+        sm.slot = slot;
+        sm.full = full;
+        sm.dt = st.inv_weight;
+        sm.contact = contact;
+        sm.move = move;
+    }
+    __syncwarp();
+    return op;
+}
+
+// What warp 0 asked for, by the whole block; returns where warp 0 goes on.
+// Out of line (and on the shared memory itself, so that its accesses are
+// known to be shared): the steps' own registers and code stay small.
+template <class LS>
+__device__ __noinline__ int block_op(int op) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    LS &sm = *reinterpret_cast<LS *>(smem_raw);
+    const BoxRun &R = sm.R;
+    typename LS::Base &rs = sm;
+    const int tid = threadIdx.x;
+    if (op == STEP_QUERY) {
+        block_query(R.box, sm.slot, Vec3{sm.dir[0], sm.dir[1], sm.dir[2]}, sm.full, sm.u.q, &sm.live);
+        if (tid == 0) apply_query(sm.st, rs, sm.u.q.out);
+        return PH_QUERIED;
+    }
+    if (op == STEP_MOVE) {
+        block_translate(R.box, sm.slot, tid < 3 ? sm.dir[tid] * sm.move : 0.0, sm.refpos);
+        return PH_MOVED;
+    }
+    if (op == STEP_REACT) {
+        commit_reactions(R, rs);
+        return PH_REACTED;
+    }
+    if (op == STEP_MERGE) {
+        commit_merge(R, rs);
+        return PH_MERGED;
+    }
+    if (op == STEP_TREE || op == STEP_LIVE) {
+        if (op == STEP_TREE) {
+            block_tree_build(R);
+            tree_cache_load(R, sm.tree);
+        }
+        live_load(R, sm.live, sm.u.q.warp_tmp);
+        return PH_MERGED;
+    }
+    commit_update(R, rs);
+    return PH_END;
+}
+
+// The shared memory of the loop: the block routines' plan, and the box's
+// record, loop state and scalars, kept on chip for the launch.
+template <class RS>
+struct LoopSmemT : RS {
+    using Base = RS;
+    BoxRun R;
+    RunState st;
+    DevScalars sc;
+    long long left;  // steps still allowed in this launch
+    const int *rec_ptr[REC_INTS];  // the integer tables of a slot's record
+};
+
+// MC steps of one box by the whole block: at most max_steps, until a stop
+// criterion, an error or the deadline.
+template <class LS>
+__device__ inline void block_steps(LS &sm, long long max_steps) {
+    unsigned t_phase = 0;
+    int phase = PH_START;  // the same in all threads
+    record_rows_init(sm);
+    if (threadIdx.x == 0) {
+        sm.stop = 0;
+        sm.left = max_steps;
+        // the criteria may have changed since the last launch; afterwards
+        // they are checked at the end of every step
+        RunState &st = sm.st;
+        if (!st.finished && st.status == ST_OK && run_finished(sm.R, st, sm.sc.n_alive)) st.finished = 1;
+    }
+    __syncthreads();
+    for (;;) {
+        if (threadIdx.x < 32) {
+            const int op = warp_steps(sm, phase, t_phase);
+            if (threadIdx.x == 0) sm.op = op;
+        }
+        __syncthreads();
+        const int op = sm.op;
+        if (op == STEP_EXIT) break;  // block-uniform
+        phase = block_op<LS>(op);
+        __syncthreads();
+    }
+}
+
+}  // namespace mcacg
