@@ -170,6 +170,9 @@ struct RunSmemT {
     unsigned long long tree_tmp;  // block reduction scratch
     double step_dt;               // this step's time increment
     double dt_indiv, step_dt_indiv;  // the moved aggregate's own time step, and its increment
+    int next_large, next_small, next_single;  // the update's work taken so far
+    int n_small;                  // aggregates listed for the threads of an update
+    int n_listed;                 // aggregates listed for the warps of an update or a contact check
     int n_moved;                  // slots whose grid cell changed in the update of all aggregates
     int moved[kMovedCap];
     TC tree;                      // top levels of the pick tree
@@ -558,6 +561,318 @@ static __device__ __noinline__ double thread_update_aggregate(const BoxRun &R, i
     return rmax;
 }
 
+// ------------------------------------------------- updates by whole warps
+// Scratch of one warp's update or contact check; the block's warps share the
+// union of the routines' plans (sm.u), as many as fit.
+constexpr int kUpdWarpMax = 32768;  // spheres of an aggregate that one warp updates (pairs pack two indices)
+constexpr int kUpdThreadMax = 4;  // spheres of an aggregate that one thread updates
+struct UpdScratch {
+    double term[8][33];  // rows of 33: lanes reading one row each meet different banks
+    int pair[64];  // pairs past the FP32 screen, i << 16 | j
+};
+// Every pair i < j of the n positions that passes the FP32 screen |p_i - p_j|
+// <= (r_i + r_j) 1.0001 + margin (of the nearest images), in (i, j) order and
+// in batches: batch(cnt) is called by all lanes with cnt <= 32 pairs in
+// W.pair[0 .. cnt). The exact tests then run on full warps (an FP64 test of
+// one row's few pairs takes as long as one of 32). n < 65536.
+template <class F>
+__device__ __forceinline__ void warp_pairs(const DevBox &b, const float4 *pos, int n, UpdScratch &W, F &&batch) {
+    const unsigned all = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    int held = 0;
+    for (int i = 0; i + 1 < n; ++i) {
+        const float4 pi_ = pos[i];
+        for (int j0 = i + 1; j0 < n; j0 += 32) {
+            const int j = j0 + lane;
+            bool hit = j < n;
+            if (hit) {
+                const float4 pj = pos[j];
+                float dx = pi_.x - pj.x, dy = pi_.y - pj.y, dz = pi_.z - pj.z;
+                dx -= b.Lf * rintf(dx * b.inv_Lf);
+                dy -= b.Lf * rintf(dy * b.inv_Lf);
+                dz -= b.Lf * rintf(dz * b.inv_Lf);
+                const float reach = (pi_.w + pj.w) * 1.0001f + b.margin_f;
+                hit = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz)) <= reach * reach;
+            }
+            const unsigned m = __ballot_sync(all, hit);
+            if (m == 0u) continue;
+            if (hit) W.pair[held + __popc(m & ((1u << lane) - 1u))] = (i << 16) | j;
+            held += __popc(m);
+            __syncwarp();
+            if (held >= 32) {
+                batch(32);
+                __syncwarp();
+                const int left = W.pair[32 + lane];
+                __syncwarp();
+                W.pair[lane] = left;
+                held -= 32;
+                __syncwarp();
+            }
+        }
+    }
+    if (held > 0) batch(held);
+    __syncwarp();
+}
+template <class RS>
+__device__ __forceinline__ int upd_warps(const RS &) {
+    return min(int(blockDim.x >> 5), int(sizeof(RS::u) / sizeof(UpdScratch)));
+}
+
+// thread_update_geometry of an aggregate of one sphere at its own centre
+// (relative position zero), by one thread: the sums have one term, so the
+// centre stays where it is and r_max, the mean radius and the mean volume
+// are the sphere's own; what is left of the FP64 work is Rg's product chain,
+// one quotient and one square root (24 instructions; the general form takes
+// about 150, and with a full update every step the update of a box of
+// monomers is bound by the FP64 pipe). Returns false when the shortcut does
+// not hold, and nothing was written.
+__device__ inline bool thread_update_monomer(const DevBox &b, int a, bool full, double *rmax, double *vol_pp,
+                                             double *volume_out, double *rg_out) {
+    const int s = b.pool_id[b.sc->pool_sel][b.agg_off[a]];
+    const double rel = S(b, SPH_RX, s), rely = S(b, SPH_RY, s), relz = S(b, SPH_RZ, s);
+    const double r = S(b, SPH_R, s), vol = S(b, SPH_VOLUME, s), sur = S(b, SPH_SURFACE, s);
+    const double x = S(b, SPH_X, s), y = S(b, SPH_Y, s), z = S(b, SPH_Z, s);
+    const double volw = full ? vol : b.sph_volw[s], volume = full ? vol : A(b, AGG_VOLUME, a);
+    const long long L = dbits(b.L);
+    if ((dbits(rel) | dbits(rely) | dbits(relz)) != 0) return false;
+    if (dbits(r) <= 0 || dbits(vol) <= 0 || dbits(sur) <= 0 || dbits(volw) <= 0 || dbits(volume) <= 0) return false;
+    if (dbits(x) < 0 || dbits(x) >= L || dbits(y) < 0 || dbits(y) >= L || dbits(z) < 0 || dbits(z) >= L) return false;
+    if (full) {
+        b.sph_volw[s] = vol;
+        A(b, AGG_VOLUME, a) = vol;
+        A(b, AGG_SURFACE, a) = sur;
+        if (b.volsurf != VS_NONE) {
+            A(b, AGG_OVERLAPPING, a) = 0.0;
+            A(b, AGG_COORDINATION_NUMBER, a) = 0.0;
+        }
+    }
+    const double rg = fp64_sqrt(fp64_div((3. / 5.) * (volw * (r * r)), volume));
+    A(b, AGG_RX, a) = 0.0;
+    A(b, AGG_RY, a) = 0.0;
+    A(b, AGG_RZ, a) = 0.0;
+    A(b, AGG_X, a) = x;
+    A(b, AGG_Y, a) = y;
+    A(b, AGG_Z, a) = z;
+    A(b, AGG_RMAX, a) = r;
+    A(b, AGG_RG, a) = rg;
+    A(b, AGG_DP, a) = __longlong_as_double(dbits(r) + (1LL << 52));  // 2 r
+    b.agg_f4[a].w = float(r);
+    *rmax = r;
+    *vol_pp = vol;
+    *volume_out = volume;
+    *rg_out = rg;
+    return true;
+}
+
+// thread_update_geometry (without 'overlap') by one warp: the spheres'
+// terms are formed a lane each and every sum runs in list order on its own
+// lane, eight sums at once; the contact pairs of "caps" and "alphas" are
+// screened in FP32 a row at a time and only those that pass are evaluated,
+// in (i, j) order. All lanes get the results.
+static __device__ __noinline__ double warp_update_geometry(const DevBox &b, int a, bool full, UpdScratch &W,
+                                                           double *vol_pp_out) {
+    const unsigned all = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int n = b.agg_n[a];
+    const int off = b.agg_off[a];
+    const int *mem = b.pool_id[b.sc->pool_sel] + off;
+    double overlapping = 0.0, coordination = 0.0;
+    AlphaSums al{0., 0., 0., 0., 0., 0.};
+    int inter = 0;
+    double *surf_w = b.work;  // by sphere index; free outside a merge
+    if (full) {
+        const bool corrected = b.volsurf != VS_NONE;
+        for (int k = lane; k < n; k += 32) {
+            b.sph_volw[mem[k]] = S(b, SPH_VOLUME, mem[k]);
+            if (corrected) surf_w[mem[k]] = S(b, SPH_SURFACE, mem[k]);
+        }
+        __syncwarp();
+        if (corrected) {
+            // (the nearest image: a superset of the pairs in contact also
+            // where positions were stored wrapped)
+            const float4 *pos = b.pool_pos[b.sc->pool_sel] + off;
+            const bool caps = b.volsurf == VS_CAPS;
+            double ov = 0.0;
+            warp_pairs(b, pos, n, W, [&](int cnt) {
+                const int ij = lane < cnt ? W.pair[lane] : 1;
+                const int si = mem[ij >> 16], sj = mem[ij & 0xffff];
+                const double ex = S(b, SPH_RX, si) - S(b, SPH_RX, sj);
+                const double ey = S(b, SPH_RY, si) - S(b, SPH_RY, sj);
+                const double ez = S(b, SPH_RZ, si) - S(b, SPH_RZ, sj);
+                const double dist = fp64_sqrt(ex * ex + ey * ey + ez * ez);
+                const double ri = S(b, SPH_R, si), rj = S(b, SPH_R, sj), rsum = ri + rj;
+                const bool touch = lane < cnt && dist <= (1. + kCoordinationEpsilon) * rsum;
+                const double c = 2.0 * fp64_div(rsum - dist, rsum);
+                SphereCaps cap{0., 0., 0., 0.};
+                if (caps && touch)
+                    cap = sphere_caps(ri, S(b, SPH_VOLUME, si), S(b, SPH_SURFACE, si), rj, S(b, SPH_VOLUME, sj),
+                                      S(b, SPH_SURFACE, sj), dist);
+                // the contacts one after another: lanes 0-3 take the caps off
+                // the two volumes and surfaces, every lane adds the overlap
+                for (unsigned m = __ballot_sync(all, touch); m != 0u; m &= m - 1u) {
+                    const int src = __ffs(m) - 1;
+                    ov += __shfl_sync(all, c, src);
+                    inter += 2;
+                    if (caps) {
+                        const int ti = __shfl_sync(all, si, src), tj = __shfl_sync(all, sj, src);
+                        const double v1 = __shfl_sync(all, cap.v1, src), s1 = __shfl_sync(all, cap.s1, src);
+                        const double v2 = __shfl_sync(all, cap.v2, src), s2 = __shfl_sync(all, cap.s2, src);
+                        if (lane < 4) {
+                            double *at = (lane & 1 ? surf_w : b.sph_volw) + (lane < 2 ? ti : tj);
+                            *at = *at - (lane == 0 ? v1 : (lane == 1 ? s1 : (lane == 2 ? v2 : s2)));
+                        }
+                        __syncwarp();
+                    } else {
+                        const double r1 = __shfl_sync(all, ri, src), r2 = __shfl_sync(all, rj, src);
+                        const double d2 = __shfl_sync(all, dist, src);
+                        alpha_add_call(al, r1, r2, d2);
+                        alpha_add_call(al, r2, r1, d2);
+                    }
+                }
+            });
+            // the clamps: a sphere's value is final once its row is done, and
+            // later rows never touch it
+            if (caps)
+                for (int k = lane; k < n; k += 32) {
+                    b.sph_volw[mem[k]] = dmax(b.sph_volw[mem[k]], 0.0);
+                    surf_w[mem[k]] = dmax(surf_w[mem[k]], 0.0);
+                }
+            __syncwarp();
+            if (inter > 0) {
+                overlapping = ov / static_cast<double>(inter);
+                coordination = static_cast<double>(inter) / static_cast<double>(n);
+            }
+        }
+    }
+    const bool plain = b.volsurf == VS_NONE;
+    // volume, surface, the weighted positions, the weighted squared radii,
+    // the radii and the plain volumes, each in list order on its lane
+    // (the next 32 spheres are loaded while the sums run)
+    double acc = 0.0;
+    {
+        double volw = 0.0, r = 0.0, sf = 0.0, x = 0.0, y = 0.0, z = 0.0, vol = 0.0;
+        auto fetch = [&](int k) {
+            if (k >= n) return;
+            const int s = mem[k];
+            volw = b.sph_volw[s];
+            r = S(b, SPH_R, s);
+            sf = !full ? 0.0 : (plain ? S(b, SPH_SURFACE, s) : surf_w[s]);
+            x = S(b, SPH_RX, s);
+            y = S(b, SPH_RY, s);
+            z = S(b, SPH_RZ, s);
+            vol = S(b, SPH_VOLUME, s);
+        };
+        fetch(lane);
+        for (int k0 = 0; k0 < n; k0 += 32) {
+            const int cnt = min(32, n - k0);
+            W.term[0][lane] = volw;
+            W.term[1][lane] = sf;
+            W.term[2][lane] = x * volw;
+            W.term[3][lane] = y * volw;
+            W.term[4][lane] = z * volw;
+            W.term[5][lane] = volw * (r * r);
+            W.term[6][lane] = r;
+            W.term[7][lane] = vol;
+            __syncwarp();
+            fetch(k0 + 32 + lane);
+            const double *v = W.term[lane & 7];
+#pragma unroll 4
+            for (int k = 0; k < cnt; ++k) acc = acc + v[k];
+            __syncwarp();
+        }
+    }
+    double volume = __shfl_sync(all, acc, 0), surface = __shfl_sync(all, acc, 1);
+    if (full) {
+        if (b.volsurf == VS_ALPHAS) alpha_finish(al, n, inter, &volume, &surface, &overlapping, &coordination);
+    } else {
+        volume = A(b, AGG_VOLUME, a);
+    }
+    const double cm = fp64_div(acc, volume);  // lanes 2-4: the centre of mass
+    const double rx = __shfl_sync(all, cm, 2), ry = __shfl_sync(all, cm, 3), rz = __shfl_sync(all, cm, 4);
+    double arg = 0.0;
+    long long rmax_bits = 0;
+    {
+        double volw = 0.0, r = 0.0, x = 0.0, y = 0.0, z = 0.0;
+        auto fetch = [&](int k) {
+            if (k >= n) return;
+            const int s = mem[k];
+            volw = b.sph_volw[s];
+            r = S(b, SPH_R, s);
+            x = S(b, SPH_RX, s);
+            y = S(b, SPH_RY, s);
+            z = S(b, SPH_RZ, s);
+        };
+        fetch(lane);
+        for (int k0 = 0; k0 < n; k0 += 32) {
+            const int cnt = min(32, n - k0);
+            const double dx = x - rx, dy = y - ry, dz = z - rz;
+            const double dc = fp64_sqrt(dx * dx + dy * dy + dz * dz);
+            const long long far = lane < cnt ? dbits(r + dc) : 0;  // below zero (an empty sphere): not taken
+            rmax_bits = far > rmax_bits ? far : rmax_bits;
+            W.term[0][lane] = volw * (dc * dc);
+            __syncwarp();
+            fetch(k0 + 32 + lane);
+#pragma unroll 4
+            for (int k = 0; k < cnt; ++k) arg = arg + W.term[0][k];
+            __syncwarp();
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const long long y = __shfl_xor_sync(all, rmax_bits, o);
+        rmax_bits = y > rmax_bits ? y : rmax_bits;
+    }
+    const double rmax = __longlong_as_double(rmax_bits);
+    const double brg = __shfl_sync(all, acc, 5), sum_r = __shfl_sync(all, acc, 6), sum_v = __shfl_sync(all, acc, 7);
+    // Rg's quotient, the mean diameter and the mean volume on lanes 0-2
+    const double num = lane == 0 ? arg + (3. / 5.) * brg : (lane == 1 ? 2 * sum_r : sum_v);
+    const double quo = fp64_div(num, lane == 0 ? volume : double(n));
+    const double rg = fp64_sqrt(fabs(__shfl_sync(all, quo, 0)));
+    *vol_pp_out = __shfl_sync(all, quo, 2);
+    const int a3 = lane < 3 ? lane : 0;
+    const double c3 = __shfl_sync(all, cm, 2 + a3);
+    if (lane < 3) {
+        const double x = wrap_position(S(b, SPH_X + lane, mem[0]) + c3, b.L);
+        A(b, AGG_X + lane, a) = x;
+        A(b, AGG_RX + lane, a) = c3;
+        reinterpret_cast<float *>(b.agg_f4 + a)[lane] = float(x);
+    }
+    if (lane == 1) A(b, AGG_DP, a) = quo;
+    if (lane == 0) {
+        A(b, AGG_RMAX, a) = rmax;
+        A(b, AGG_RG, a) = rg;
+        b.agg_f4[a].w = float(rmax);
+        if (full) {
+            A(b, AGG_VOLUME, a) = volume;
+            A(b, AGG_SURFACE, a) = surface;
+            if (!plain) {
+                A(b, AGG_OVERLAPPING, a) = overlapping;
+                A(b, AGG_COORDINATION_NUMBER, a) = coordination;
+            }
+        }
+    }
+    __syncwarp();
+    return rmax;
+}
+// thread_update_aggregate by one warp.
+__device__ inline double warp_update_aggregate(const BoxRun &R, int a, bool full, UpdScratch &W) {
+    const DevBox &b = R.box;
+    double vol_pp = 0.0;
+    const double rmax = warp_update_geometry(b, a, full, W, &vol_pp);
+    const double dp = A(b, AGG_DP, a);
+    const float4 v = physics_f32(R.phys, float(half_of(dp)), float(A(b, AGG_VOLUME, a)), float(vol_pp));
+    const double dgdp = fp64_div(A(b, AGG_RG, a), half_of(dp));
+    if ((threadIdx.x & 31) == 0) {
+        A(b, AGG_F_AGG, a) = double(v.x);
+        A(b, AGG_D_M, a) = double(v.y);
+        A(b, AGG_TIME_STEP, a) = double(v.z);
+        A(b, AGG_LPM, a) = double(v.w);
+        A(b, AGG_DG_OVER_DP, a) = dgdp;
+    }
+    __syncwarp();
+    return rmax;
+}
+
 // The pick tree from the time steps: the scale from the largest weight and
 // the live count, leaves of the live slots (0 elsewhere), then each level
 // from the one below, and the total into the loop state. The FP64 weights
@@ -577,15 +892,24 @@ static __device__ __noinline__ void block_tree_build(const BoxRun &R) {
     for (int a = tid; a < R.tree_len[0]; a += NT) {
         double w = 0.0;
         if (a < b.nslots && b.agg_n[a] > 0) {
-            w = 1.0 / A(b, AGG_TIME_STEP, a);
+            w = fp64_div(1.0, A(b, AGG_TIME_STEP, a));
             ++live;
         }
         const unsigned long long bits = static_cast<unsigned long long>(__double_as_longlong(w));
         R.tree[R.tree_off[0] + a] = bits;
         mb = bits > mb ? bits : mb;
     }
-    atomicMax(&max_bits, mb);
-    atomicAdd(&n_live, live);
+    // one atomic a warp: 512 threads' 64-bit maxima on one shared word took
+    // some 50 000 cycles, a third of a growing box's update
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long other = __shfl_xor_sync(0xffffffffu, mb, o);
+        mb = other > mb ? other : mb;
+    }
+    live = __reduce_add_sync(0xffffffffu, live);
+    if ((tid & 31) == 0) {
+        atomicMax(&max_bits, mb);
+        atomicAdd(&n_live, live);
+    }
     __syncthreads();
     if (tid == 0) {
         // n_live * max weight * scale < 2^62
@@ -635,20 +959,82 @@ __device__ inline void block_update_all(const BoxRun &R, RS &sm, bool full) {
     const DevBox &b = R.box;
     const int tid = threadIdx.x, NT = blockDim.x;
     double rmax_d = 0.0;
-    if (tid == 0) sm.n_moved = 0;
+    if (tid == 0) {
+        sm.n_moved = 0;
+        sm.n_listed = 0;
+        sm.n_small = 0;
+        sm.next_large = sm.next_small = sm.next_single = 0;
+    }
     __syncthreads();
-    for (int a = tid; a < b.nslots; a += NT) {
-        if (b.agg_n[a] == 0) continue;
-        const double rm = thread_update_aggregate(R, a, full);
-        rmax_d = dmax(rmax_d, rm);
-        // the centre moves a little when spheres grow unevenly: note the
-        // slots whose Verlet or fine cell changed
+    int *list = b.cand_slot, *small = b.cand_order;  // free outside a query
+    // the centre moves a little when spheres grow unevenly: note the slots
+    // whose Verlet or fine cell changed
+    auto note_cell = [&](int a) {
         const Vec3 pa = agg_pos(b, a);
         if (cell_of(b, pa) != b.agg_cell[a] || (b.fine_div > 0 && fine_cell_of(b, pa) != b.fine_cell[a])) {
             const int k = atomicAdd(&sm.n_moved, 1);
             if (k < kMovedCap) sm.moved[k] = a;
         }
+    };
+    for (int a = tid; a < b.nslots; a += NT) {
+        const int n = b.agg_n[a];
+        if (n > kUpdThreadMax && n < kUpdWarpMax) list[atomicAdd(&sm.n_listed, 1)] = a;
+        else if (n > 1) small[atomicAdd(&sm.n_small, 1)] = a;
     }
+    __syncthreads();
+    // the warps take the work in order of length: aggregates of many spheres
+    // (a warp each), of a few (a thread each), then 32 slots of single
+    // spheres at a time, so that the long chains run beside the many short
+    // ones (whose FP64 work fills the pipes)
+    const int lane = tid & 31, wid = tid >> 5, nw = upd_warps(sm);
+    auto next = [&](int *counter, int by) {
+        int k = 0;
+        if (lane == 0) k = atomicAdd(counter, by);
+        return __shfl_sync(0xffffffffu, k, 0);
+    };
+    if (wid < nw) {
+        UpdScratch &W = reinterpret_cast<UpdScratch *>(&sm.u)[wid];
+        for (int k = next(&sm.next_large, 1); k < sm.n_listed; k = next(&sm.next_large, 1)) {
+            const double rm = warp_update_aggregate(R, list[k], full, W);
+            rmax_d = dbits(rm) > dbits(rmax_d) ? rm : rmax_d;
+            if (lane == 0) note_cell(list[k]);
+        }
+    }
+    for (int k = next(&sm.next_small, 32); k < sm.n_small; k = next(&sm.next_small, 32)) {
+        if (k + lane >= sm.n_small) continue;
+        const int a = small[k + lane];
+        const double rm = thread_update_aggregate(R, a, full);
+        rmax_d = dbits(rm) > dbits(rmax_d) ? rm : rmax_d;
+        note_cell(a);
+    }
+    __syncwarp();
+    for (int k = next(&sm.next_single, 32); k < b.nslots; k = next(&sm.next_single, 32)) {
+        const int a = k + lane;
+        if (a >= b.nslots || b.agg_n[a] != 1) continue;
+        double rm, vol_pp, volume, rg;
+        const double x0 = A(b, AGG_X, a), y0 = A(b, AGG_Y, a), z0 = A(b, AGG_Z, a);
+        if (thread_update_monomer(b, a, full, &rm, &vol_pp, &volume, &rg)) {
+            const float V = float(volume);
+            const float4 v = physics_f32(R.phys, b.agg_f4[a].w, V, dbits(vol_pp) == dbits(volume) ? V : float(vol_pp));
+            A(b, AGG_F_AGG, a) = double(v.x);
+            A(b, AGG_D_M, a) = double(v.y);
+            A(b, AGG_TIME_STEP, a) = double(v.z);
+            A(b, AGG_LPM, a) = double(v.w);
+            A(b, AGG_DG_OVER_DP, a) = fp64_div(rg, rm);
+            // the centre is where it was, unless the record had another
+            if (((dbits(x0) ^ dbits(A(b, AGG_X, a))) | (dbits(y0) ^ dbits(A(b, AGG_Y, a))) |
+                 (dbits(z0) ^ dbits(A(b, AGG_Z, a)))) != 0) {
+                const Vec3 pa = agg_pos(b, a);
+                b.agg_f4[a] = make_float4(float(pa.x), float(pa.y), float(pa.z), float(rm));
+                note_cell(a);
+            }
+        } else {
+            rm = thread_update_aggregate(R, a, full);
+            note_cell(a);
+        }
+        rmax_d = dbits(rm) > dbits(rmax_d) ? rm : rmax_d;
+    }
+    __syncwarp();
     // block max of r_max (bits of a non-negative double order like integers)
     unsigned long long bits = static_cast<unsigned long long>(__double_as_longlong(rmax_d));
     for (int o = 16; o > 0; o >>= 1) {
@@ -684,10 +1070,14 @@ __device__ inline void block_update_one_or_all(const BoxRun &R, RS &sm, int slot
         return;
     }
     const DevBox &b = R.box;
-    if (threadIdx.x == 0) {
-        const double rm = thread_update_aggregate(R, slot, full);
-        if (rm > b.sc->maxradius) b.sc->maxradius = rm;
-        regrid(b, slot, agg_pos(b, slot));
+    if (threadIdx.x < 32) {
+        const double rm = b.agg_n[slot] < kUpdWarpMax
+                              ? warp_update_aggregate(R, slot, full, *reinterpret_cast<UpdScratch *>(&sm.u))
+                              : (threadIdx.x == 0 ? thread_update_aggregate(R, slot, full) : 0.0);
+        if (threadIdx.x == 0) {
+            if (rm > b.sc->maxradius) b.sc->maxradius = rm;
+            regrid(b, slot, agg_pos(b, slot));
+        }
     }
     __syncthreads();
     if (threadIdx.x < 32) {
@@ -995,6 +1385,124 @@ __device__ inline void block_split_slot(const BoxRun &R, RS &sm, int a) {
     __syncthreads();
 }
 
+// The contact networks of the m listed aggregates (all threads): apart[k] is
+// set to 1 where aggregate list[k] falls into more than one part, or where
+// this cannot tell (more contacts than block_split_slot's pair scratch
+// holds), else to 0. The contacts are block_split_slot's: an FP32 screen of
+// the member positions, then the exact test, which only pairs within the
+// screen's margin of touching need. The rows of all aggregates' pair
+// triangles are handed to the warps in turn, so that one large aggregate
+// occupies them all; the forests stand in one array over the rows, in shared
+// memory up to kForestRows. A block call for every aggregate was 13 barriers
+// and a dozen rounds of loads each, for an answer that is nearly always
+// "connected".
+constexpr int kForestRows = 2048;
+struct ForestPair {
+    int i, j, shift;  // rows; pool place less row
+};
+template <class RS>
+__device__ inline void block_connected(const BoxRun &R, RS &sm, const long long *list, int m, int *apart) {
+    const DevBox &b = R.box;
+    const unsigned all = 0xffffffffu;
+    const int tid = threadIdx.x, NT = blockDim.x, lane = tid & 31, wid = tid >> 5;
+    int *first = b.cand_slot;  // first row of each listed aggregate, m + 1 entries
+    const int *pool = b.pool_id[b.sc->pool_sel];
+    const float4 *pp = b.pool_pos[b.sc->pool_sel];
+    for (int k = tid; k <= m; k += NT) first[k] = k < m ? b.agg_n[list[k]] : 0;
+    if (tid == 0) {
+        sm.n_listed = 0;
+        sm.n_small = 0;
+    }
+    __syncthreads();
+    const int rows = block_scan_global(first, m + 1, sm.u.m.warp_tmp);
+    __syncthreads();
+    int *shared = reinterpret_cast<int *>(&sm.u);
+    static_assert(sizeof(RS::u) >= sizeof(int) * kForestRows + 64 * sizeof(ForestPair), "room for one warp");
+    const int nw = min(NT >> 5, int((sizeof(RS::u) - sizeof(int) * kForestRows) / (64 * sizeof(ForestPair))));
+    int *parent = rows <= kForestRows ? shared : b.row_cnt;
+    ForestPair *held_pairs = reinterpret_cast<ForestPair *>(shared + kForestRows) + 64 * min(wid, nw - 1);
+    for (int r = tid; r < rows; r += NT) parent[r] = r;
+    __syncthreads();
+    bool ok = true;
+    int pairs = 0;
+    if (wid < nw) {
+        int held = 0, k = 0, base = 0, n = 0, off = 0;
+        // the exact test of cnt held pairs, and their union
+        auto batch = [&](int cnt) {
+            bool hit = lane < cnt;
+            if (hit) {
+                const ForestPair f = held_pairs[lane];
+                const int si = pool[f.i + f.shift], sj = pool[f.j + f.shift];
+                const double dx = wrap_distance(S(b, SPH_X, si) - S(b, SPH_X, sj), b.L);
+                const double dy = wrap_distance(S(b, SPH_Y, si) - S(b, SPH_Y, sj), b.L);
+                const double dz = wrap_distance(S(b, SPH_Z, si) - S(b, SPH_Z, sj), b.L);
+                const double d2 = dx * dx + dy * dy + dz * dz, sum = S(b, SPH_R, si) + S(b, SPH_R, sj);
+                hit = d2 - sum * sum <= kContactEpsilon;  // spheres_in_contact
+                if (hit) ok = uf_unite(parent, f.i, f.j, rows) && ok;
+            }
+            pairs += __popc(__ballot_sync(all, hit));
+        };
+        for (int row = wid; row < rows; row += nw) {
+            while (row >= first[k + 1]) ++k;  // rows ascend
+            if (base != first[k] || n == 0) {
+                base = first[k];
+                n = first[k + 1] - base;
+                off = b.agg_off[list[k]];
+            }
+            const int i = row - base;
+            const float4 pi_ = pp[off + i];
+            for (int j0 = i + 1; j0 < n; j0 += 32) {
+                const int j = j0 + lane;
+                bool hit = false, sure = false;
+                if (j < n) {
+                    const float4 pj = pp[off + j];
+                    const float dx = pi_.x - pj.x, dy = pi_.y - pj.y, dz = pi_.z - pj.z;
+                    const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
+                    const float reach = (pi_.w + pj.w) * 1.0001f + b.margin_f;
+                    const float inner = (pi_.w + pj.w) * 0.9999f - b.margin_f;
+                    hit = d2 <= reach * reach;
+                    sure = inner > 0.f && d2 <= inner * inner;
+                }
+                // overlapping by more than the margin: in contact without the
+                // exact test
+                pairs += __popc(__ballot_sync(all, sure));
+                if (sure) ok = uf_unite(parent, row, base + j, rows) && ok;
+                hit = hit && !sure;
+                const unsigned mk = __ballot_sync(all, hit);
+                if (mk == 0u) continue;
+                if (hit) held_pairs[held + __popc(mk & ((1u << lane) - 1u))] = ForestPair{row, base + j, off - base};
+                held += __popc(mk);
+                __syncwarp();
+                if (held >= 32) {
+                    batch(32);
+                    __syncwarp();
+                    const ForestPair left = held_pairs[32 + lane];
+                    __syncwarp();
+                    held_pairs[lane] = left;
+                    held -= 32;
+                    __syncwarp();
+                }
+            }
+        }
+        if (held > 0) batch(held);
+        if (lane == 0) atomicAdd(&sm.n_small, pairs);
+        if (!ok) sm.n_listed = 1;
+    }
+    __syncthreads();
+    const int lost = sm.n_listed != 0 || sm.n_small > b.pair_cap;
+    for (int k = tid; k < m; k += NT) apart[k] = lost;
+    __syncthreads();
+    for (int row = tid; row < rows; row += NT) {
+        int lo = 0, hi = m - 1;  // the aggregate of this row: last first <= row
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (first[mid] <= row) lo = mid; else hi = mid - 1;
+        }
+        if (uf_find(parent, row) != uf_find(parent, first[lo])) apart[lo] = 1;
+    }
+    __syncthreads();
+}
+
 // The oxidation of a step (all threads), after the spheres shrank: removals
 // and disappearances, then splits -- of the moved aggregate (slot >= 0, the
 // individual mode, calcul.cpp:159-163) or of every aggregate (calcul.cpp:
@@ -1024,8 +1532,21 @@ __device__ __noinline__ void block_oxidize(const BoxRun &R, RS &sm, int slot) {
     for (int a = tid; a < b.nslots; a += NT)
         if (b.agg_n[a] >= 2) list[flag[a]] = a;
     __syncthreads();
-    for (int k = 0; k < m; ++k) {
-        block_split_slot(R, sm, int(list[k]));
+    // the aggregates that fall apart are left to the block's split, one after
+    // another in slot order
+    int *apart = b.cand_prefix;
+    block_connected(R, sm, list, m, apart);
+    // a split may use the lists' scratch: the slots to visit move out of it
+    if (tid == 0) {
+        int v = 0;
+        for (int k = 0; k < m; ++k)
+            if (apart[k]) flag[v++] = int(list[k]);
+        sm.n_listed = v;
+    }
+    __syncthreads();
+    const int visit = sm.n_listed;
+    for (int k = 0; k < visit; ++k) {
+        block_split_slot(R, sm, flag[k]);
         if (b.sc->status != ST_OK) break;
     }
     __syncthreads();
