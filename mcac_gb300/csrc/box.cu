@@ -3,7 +3,9 @@
 
 #include <algorithm>
 #include <cstring>
+#include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -439,6 +441,67 @@ __global__ void __launch_bounds__(kScanThreads) k_boxes(const DevBox *boxes, con
     if ((OP == OP_PACK_RANKS || OP == OP_PACK) && arg.a < 0) return;  // block-uniform
     box_op<OP>(b, arg, (blockIdx.x % per_box) * blockDim.x + threadIdx.x, per_box * blockDim.x);
 }
+// Many copies in one launch, between device memory and page-locked host
+// memory in either direction. A batch of small boxes is thousands of small
+// arrays, and a copy of the driver's takes about 2 us each whatever its size
+// (2000 boxes of 1000 monomers: 12 000 copies, 29 ms up and 27 ms down for
+// 0.53 GB each way; with this kernel 8.7 and 9.3 ms, allocations included;
+// the 512-box ensemble 10.8-43 and 10.4-43 ms before, 5.5 and 12.2 ms now).
+// It moves what the copy engines do, 211 GB/s up and 193 GB/s down, from 152
+// blocks on. The pieces are cut into chunks of kPieceChunk bytes, which the
+// blocks take in turn; 'first' is the first chunk of each piece.
+struct CopyPiece {
+    const char *src;
+    char *dst;
+    unsigned long long bytes;  // a multiple of 8; both ends 8-byte aligned
+};
+constexpr unsigned long long kPieceChunk = 32768;
+__global__ void __launch_bounds__(256) k_copy_pieces(const CopyPiece *pieces, const int *first, int n) {
+    const int total = first[n];
+    for (int c = blockIdx.x; c < total; c += gridDim.x) {
+        int lo = 0, hi = n - 1;  // the piece of chunk c: last first <= c
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (first[mid] <= c) lo = mid; else hi = mid - 1;
+        }
+        const CopyPiece p = pieces[lo];
+        const unsigned long long off = (unsigned long long)(c - first[lo]) * kPieceChunk;
+        const int bytes = int(min(kPieceChunk, p.bytes - off));
+        const char *src = p.src + off;
+        char *dst = p.dst + off;
+        if (((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0) {
+            // eight loads in flight a thread: host memory is 1-2 us away
+            const int m = bytes >> 4;
+            const int4 *s4 = reinterpret_cast<const int4 *>(src);
+            int4 *d4 = reinterpret_cast<int4 *>(dst);
+            for (int i0 = threadIdx.x; i0 < m; i0 += 8 * 256) {
+                int4 v[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (i0 + u * 256 < m) v[u] = s4[i0 + u * 256];
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (i0 + u * 256 < m) d4[i0 + u * 256] = v[u];
+            }
+            if ((bytes & 8) && threadIdx.x == 0)
+                reinterpret_cast<int2 *>(dst)[2 * m] = reinterpret_cast<const int2 *>(src)[2 * m];
+        } else {
+            const int m = bytes >> 3;
+            const int2 *s2 = reinterpret_cast<const int2 *>(src);
+            int2 *d2 = reinterpret_cast<int2 *>(dst);
+            for (int i0 = threadIdx.x; i0 < m; i0 += 8 * 256) {
+                int2 v[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (i0 + u * 256 < m) v[u] = s2[i0 + u * 256];
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (i0 + u * 256 < m) d2[i0 + u * 256] = v[u];
+            }
+        }
+    }
+}
+
 // the scalars of many boxes, gathered for one copy to the host
 __global__ void k_gather_scalars(const DevBox *boxes, int n, DevScalars *out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -456,6 +519,67 @@ bool cuda_ok(cudaError_t e, std::string *err, const char *what) {
 struct OutBuffers {
     QueryOut query;
     MergeOut merge;
+};
+
+// Page-locked host blocks handed out by the library (mcacg_host_alloc), so
+// that their arrays are known without a question to the driver.
+std::mutex g_pinned_lock;
+std::map<uintptr_t, size_t> g_pinned;  // start -> bytes
+
+// The address at which kernels reach 'bytes' of host memory at p when they lie
+// in such a block (portable memory has one address on every device), else
+// null.
+const char *device_view(const void *p, size_t bytes) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    {
+        std::lock_guard<std::mutex> hold(g_pinned_lock);
+        auto it = g_pinned.upper_bound(a);
+        if (it != g_pinned.begin()) {
+            --it;
+            if (a >= it->first && a + bytes <= it->first + it->second) return static_cast<const char *>(p);
+        }
+    }
+    return nullptr;
+}
+
+// Copies of many pieces by one kernel (k_copy_pieces).
+class PieceCopies {
+  public:
+    void add(const void *src, void *dst, size_t bytes) {
+        if (bytes == 0) return;
+        first_.push_back(int(chunks_));
+        pieces_.push_back(CopyPiece{static_cast<const char *>(src), static_cast<char *>(dst), bytes});
+        chunks_ += (bytes + kPieceChunk - 1) / kPieceChunk;
+        aligned_ = aligned_ && bytes % 8 == 0 && reinterpret_cast<uintptr_t>(src) % 8 == 0 &&
+                   reinterpret_cast<uintptr_t>(dst) % 8 == 0;
+    }
+    // the kernel can do them: every end 8-byte aligned, chunk numbers in range
+    bool ok() const { return aligned_ && chunks_ < (1ull << 31) - 1; }
+    size_t table_bytes() const {
+        return (sizeof(CopyPiece) * pieces_.size() + 255) / 256 * 256 + sizeof(int) * (pieces_.size() + 1);
+    }
+    // 'table' is table_bytes() of device memory; the vectors must live until
+    // the stream has passed the upload
+    bool launch(char *table, cudaStream_t s, int n_sm, std::string *err) {
+        if (pieces_.empty()) return true;
+        first_.push_back(int(chunks_));
+        CopyPiece *p = reinterpret_cast<CopyPiece *>(table);
+        int *f = reinterpret_cast<int *>(table + (sizeof(CopyPiece) * pieces_.size() + 255) / 256 * 256);
+        if (!cuda_ok(cudaMemcpyAsync(p, pieces_.data(), sizeof(CopyPiece) * pieces_.size(), cudaMemcpyHostToDevice, s),
+                     err, "upload") ||
+            !cuda_ok(cudaMemcpyAsync(f, first_.data(), sizeof(int) * first_.size(), cudaMemcpyHostToDevice, s), err,
+                     "upload"))
+            return false;
+        const int grid = int(std::min<unsigned long long>(chunks_, 4ull * unsigned(n_sm)));
+        k_copy_pieces<<<grid, 256, 0, s>>>(p, f, int(pieces_.size()));
+        return cuda_ok(cudaGetLastError(), err, "k_copy_pieces");
+    }
+
+  private:
+    std::vector<CopyPiece> pieces_;
+    std::vector<int> first_;
+    unsigned long long chunks_ = 0;
+    bool aligned_ = true;
 };
 
 }  // namespace
@@ -491,6 +615,15 @@ StateView view_of(const HostState &st, std::vector<int> *compact) {
         v.members = compact->data();
     }
     return v;
+}
+
+void pinned_block_add(void *p, size_t bytes) {
+    std::lock_guard<std::mutex> hold(g_pinned_lock);
+    g_pinned[reinterpret_cast<uintptr_t>(p)] = bytes;
+}
+void pinned_block_remove(void *p) {
+    std::lock_guard<std::mutex> hold(g_pinned_lock);
+    g_pinned.erase(reinterpret_cast<uintptr_t>(p));
 }
 
 int DeviceBox::create(const HostState &st, void *stream, DeviceBox **out, std::string *err) {
@@ -677,6 +810,26 @@ bool upload_state(const DevBox &b, const StateView &st, cudaStream_t s, std::str
            put(b.sc, &sc, sizeof(sc));
 }
 
+// The same as pieces of one kernel's copies, the scalars from 'sc' (device
+// memory). False when an array is not page-locked.
+bool upload_pieces(const DevBox &b, const StateView &st, const DevScalars *sc, PieceCopies *out) {
+    const size_t iw = st.wide ? 8 : 4;
+    const LoadStage in = load_stage(b, st.wide ? 1 : 0, st.dead_slots ? 1 : 0);
+    bool ok = true;
+    auto put = [&](const void *dst, const void *src, size_t bytes) {
+        const char *from = device_view(src, bytes);
+        ok = ok && from != nullptr;
+        if (ok) out->add(from, const_cast<void *>(dst), bytes);
+    };
+    put(b.sph, st.sph, sizeof(double) * 9 * size_t(st.ns));
+    put(b.agg, st.agg, sizeof(double) * 21 * size_t(st.nslots));
+    put(in.label, st.sph_slot, iw * size_t(st.ns));
+    put(in.members, st.members, iw * size_t(st.ns));
+    put(in.count, st.agg_n, iw * size_t(st.nslots));
+    out->add(sc, b.sc, sizeof(DevScalars));
+    return ok;
+}
+
 const char *load_error_text(int code) {
     switch (code) {
         case LOAD_LABEL: return "sphere label out of range";
@@ -688,12 +841,18 @@ const char *load_error_text(int code) {
 }
 
 // blocks per box of the many-box kernels: enough to fill the GPU
+int sm_count();
 int blocks_per_box(int n_boxes, int max_items) {
+    const int n_sm = sm_count();
+    const int want = (8 * n_sm + n_boxes - 1) / std::max(1, n_boxes);
+    return std::max(1, std::min({want, 256, (max_items + 255) / 256}));
+}
+
+int sm_count() {
     int dev = 0, n_sm = 0;
     cudaGetDevice(&dev);
     if (cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n_sm <= 0) n_sm = 152;
-    const int want = (8 * n_sm + n_boxes - 1) / std::max(1, n_boxes);
-    return std::max(1, std::min({want, 256, (max_items + 255) / 256}));
+    return n_sm;
 }
 
 // A few streams that share the copies of many boxes (several copy engines
@@ -747,6 +906,12 @@ class CopyStreams {
     cudaEvent_t ev_ = nullptr;
 };
 constexpr int kCopyStreams = 4;
+// one kernel's copies (k_copy_pieces) from this many boxes on (below, the few
+// copies cost less than its table), of less than this many bytes of device
+// memory each (above, the 2 us a copy do not matter and the copy engines
+// leave the SMs free)
+constexpr int kPieceMinBoxes = 16;
+constexpr size_t kPieceMaxBox = size_t(64) << 20;
 
 }  // namespace
 
@@ -847,20 +1012,56 @@ int DeviceBox::create_many(const std::vector<StateView> &views, void *stream,
     }
     std::shared_ptr<void> shared(arena, [](void *p) { cudaFree(p); });
     for (int i = 0; i < n; ++i) carve_fixed(plans[size_t(i)], arena + off[size_t(i)]);
-    // the copies, spread over a few streams, then joined into the main one
-    CopyStreams copies(kCopyStreams);
-    if (!copies.fork(s)) {
-        if (err) *err = "copy streams";
-        return ST_CUDA;
-    }
-    for (int i = 0; i < n; ++i)
-        if (!upload_state(plans[size_t(i)], views[size_t(i)], copies.at(size_t(i), s), err)) {
-            if (err) *err = "box " + std::to_string(i) + ": " + *err;
-            return ST_CUDA;  // the copy streams are synchronised on the way out
+    // the copies: one kernel over all arrays where they are page-locked and
+    // mostly small; else spread over a few streams, then joined into the main
+    // one
+    static_assert(sizeof(DevScalars) % 8 == 0, "copied in words of 8 bytes");
+    PieceCopies pieces;
+    std::vector<DevScalars> start(static_cast<size_t>(n));
+    char *copy_tmp = nullptr;
+    std::unique_ptr<char, void (*)(char *)> copy_owner(nullptr, [](char *p) { cudaFree(p); });
+    const bool one_kernel = n >= kPieceMinBoxes && off[size_t(n)] / size_t(n) < kPieceMaxBox && [&] {
+        const size_t sc_bytes = (sizeof(DevScalars) * size_t(n) + 255) & ~size_t(255);
+        // room for the table of 6 pieces a box and their chunk numbers
+        const size_t room = sc_bytes + 6 * (sizeof(CopyPiece) + sizeof(int)) * size_t(n) + 1024;
+        if (cudaMalloc((void **)&copy_tmp, room) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
         }
-    if (!copies.join(s)) {
-        if (err) *err = "copy streams";
-        return ST_CUDA;
+        copy_owner.reset(copy_tmp);
+        for (int i = 0; i < n; ++i) {
+            start[size_t(i)] = DevScalars{};
+            start[size_t(i)].maxradius = views[size_t(i)].maxradius;
+            start[size_t(i)].time = views[size_t(i)].time;
+            if (!upload_pieces(plans[size_t(i)], views[size_t(i)], reinterpret_cast<DevScalars *>(copy_tmp) + i,
+                               &pieces))
+                return false;
+        }
+        return pieces.ok();
+    }();
+    if (one_kernel) {
+        const size_t sc_bytes = (sizeof(DevScalars) * size_t(n) + 255) & ~size_t(255);
+        if (!cuda_ok(cudaMemcpyAsync(copy_tmp, start.data(), sizeof(DevScalars) * size_t(n), cudaMemcpyHostToDevice, s),
+                     err, "upload") ||
+            !pieces.launch(copy_tmp + sc_bytes, s, sm_count(), err)) {
+            cudaStreamSynchronize(s);
+            return ST_CUDA;
+        }
+    } else {
+        CopyStreams copies(kCopyStreams);
+        if (!copies.fork(s)) {
+            if (err) *err = "copy streams";
+            return ST_CUDA;
+        }
+        for (int i = 0; i < n; ++i)
+            if (!upload_state(plans[size_t(i)], views[size_t(i)], copies.at(size_t(i), s), err)) {
+                if (err) *err = "box " + std::to_string(i) + ": " + *err;
+                return ST_CUDA;  // the copy streams are synchronised on the way out
+            }
+        if (!copies.join(s)) {
+            if (err) *err = "copy streams";
+            return ST_CUDA;
+        }
     }
     parallel_for(n, [&](int i) { plan_grids(views[size_t(i)], plans[size_t(i)]); });
     std::vector<size_t> goff(static_cast<size_t>(n) + 1, 0);
@@ -1565,27 +1766,55 @@ int DeviceBox::store_many(const std::vector<DeviceBox *> &boxes, const std::vect
     k_boxes<OP_PACK_RANKS><<<n, kScanThreads, 0, s>>>(dboxes, dargs, n, 1);
     k_boxes<OP_PACK><<<n * per, 256, 0, s>>>(dboxes, dargs, n, per);
     if (!cuda_ok(cudaGetLastError(), err, "store")) return ST_CUDA;
-    // the copies, spread over a few streams after the packing
-    CopyStreams copies(kCopyStreams);
-    if (!copies.fork(s)) {
-        if (err) *err = "copy streams";
-        return ST_CUDA;
-    }
-    cudaStream_t cs = s;
-    auto get = [&](void *dst, const void *src, size_t bytes) {
-        return cuda_ok(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, cs), err, "store");
+    // the copies after the packing: one kernel where the arrays are
+    // page-locked and mostly small, else spread over a few streams
+    auto each = [&](auto &&get) {
+        for (int i = 0; i < n; ++i) {
+            const int na = args[size_t(i)].a;
+            if (na < 0) continue;
+            const DevBox &b = host_boxes[size_t(i)];
+            const PackStage ps = pack_stage(b, na, args[size_t(i)].b);
+            mcacg_state *o = outs[size_t(i)];
+            if (!(get(i, o->spheres, b.sph, sizeof(double) * 9 * size_t(b.ns)) &&
+                  get(i, o->sphere_label, ps.label, 8 * size_t(b.ns)) &&
+                  get(i, o->aggregates, ps.agg, 168 * size_t(na)) &&
+                  get(i, o->n_spheres_per_aggregate, ps.count, 8 * size_t(na)) &&
+                  get(i, o->members, ps.members, 8 * size_t(b.ns))))
+                return false;
+        }
+        return true;
     };
-    for (int i = 0; i < n; ++i) {
-        const int na = args[size_t(i)].a;
-        if (na < 0) continue;
-        const DevBox &b = host_boxes[size_t(i)];
-        const PackStage ps = pack_stage(b, na, args[size_t(i)].b);
-        mcacg_state *o = outs[size_t(i)];
-        cs = copies.at(size_t(i), s);
-        if (!(get(o->spheres, b.sph, sizeof(double) * 9 * size_t(b.ns)) &&
-              get(o->sphere_label, ps.label, 8 * size_t(b.ns)) && get(o->aggregates, ps.agg, 168 * size_t(na)) &&
-              get(o->n_spheres_per_aggregate, ps.count, 8 * size_t(na)) &&
-              get(o->members, ps.members, 8 * size_t(b.ns))))
+    PieceCopies pieces;
+    size_t total_bytes = 0;
+    for (const DevBox &b : host_boxes) total_bytes += 88 * size_t(b.ns);
+    char *copy_tmp = nullptr;
+    std::unique_ptr<char, void (*)(char *)> copy_owner(nullptr, [](char *p) { cudaFree(p); });
+    bool one_kernel = n >= kPieceMinBoxes && total_bytes / size_t(n) < kPieceMaxBox / 8;
+    one_kernel = one_kernel && each([&](int, void *dst, const void *src, size_t bytes) {
+                     char *to = const_cast<char *>(device_view(dst, bytes));
+                     if (to != nullptr) pieces.add(src, to, bytes);
+                     return to != nullptr;
+                 }) && pieces.ok();
+    if (one_kernel && cudaMalloc((void **)&copy_tmp, pieces.table_bytes()) != cudaSuccess) {
+        cudaGetLastError();
+        one_kernel = false;
+    }
+    copy_owner.reset(copy_tmp);
+    CopyStreams copies(one_kernel ? 0 : kCopyStreams);
+    if (one_kernel) {
+        if (!pieces.launch(copy_tmp, s, sm_count(), err)) {
+            cudaStreamSynchronize(s);
+            return ST_CUDA;
+        }
+    } else {
+        if (!copies.fork(s)) {
+            if (err) *err = "copy streams";
+            return ST_CUDA;
+        }
+        if (!each([&](int i, void *dst, const void *src, size_t bytes) {
+                return cuda_ok(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, copies.at(size_t(i), s)), err,
+                               "store");
+            }))
             return ST_CUDA;
     }
     if (!copies.join(s) || !cuda_ok(cudaStreamSynchronize(s), err, "sync")) return ST_CUDA;

@@ -773,13 +773,17 @@ int mcacg_host_alloc(int64_t bytes, void **ptr) {
             *ptr = nullptr;
             return fail(mcacg::ST_CUDA, std::string("cudaHostAlloc: ") + cudaGetErrorString(e));
         }
+        mcacg::pinned_block_add(*ptr, size_t(bytes));
         return 0;
     });
 }
 
 int mcacg_host_free(void *ptr) {
     return guarded([&] {
-        if (ptr) cudaFreeHost(ptr);
+        if (ptr) {
+            mcacg::pinned_block_remove(ptr);
+            cudaFreeHost(ptr);
+        }
         return 0;
     });
 }

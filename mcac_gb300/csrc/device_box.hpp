@@ -112,6 +112,11 @@ struct MergeResult {
     double maxradius;
 };
 
+// Page-locked host blocks the library handed out (mcacg_host_alloc): states
+// in them are copied by kernels of the library's own.
+void pinned_block_add(void *p, size_t bytes);
+void pinned_block_remove(void *p);
+
 // Merged aggregates of at least this many spheres find their contact pairs
 // on a hashed cell grid, smaller ones by testing all pairs (the same pairs
 // either way). Process-wide; read when a box is created. Default 2048.
