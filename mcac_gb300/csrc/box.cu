@@ -13,6 +13,7 @@
 #include "device_box.hpp"
 #include "host_parallel.hpp"
 #include "merge.cuh"
+#include "warp_query.cuh"
 
 #include <atomic>
 
@@ -27,11 +28,59 @@ int set_merge_grid_min(int n) { return g_merge_grid_min.exchange(n); }
 
 
 // ------------------------------------------------------------------ kernels
+// A query by one warp into *out (lane 0 writes it); false when it is the
+// block's (then *out is untouched).
+template <class WS>
+__device__ __forceinline__ bool warp_query_out(const DevBox &b, const DevScalars *sc, WS &W, const RecRows &rows, int src,
+                                               Vec3 dir, double dist, QueryOut *out) {
+    const int lane = threadIdx.x & 31;
+    const unsigned t0 = clock_lo();
+    const WarpRec rec = load_record(rows, src);
+    WarpAnswer o;
+    if (!warp_query(b, sc, W, static_cast<const int *>(nullptr), 0, src, rec,
+                    lane == 0 ? dir.x : (lane == 1 ? dir.y : dir.z), dist, o))
+        return false;
+    const int n_mov = shfl_i(rec.i, REC_N);
+    if (lane == 0) {
+        QueryOut r;
+        r.distance = o.distance;
+        r.moving_sphere = o.ms;
+        r.other_sphere = o.os;
+        r.other_slot = o.oslot;
+        r.status = o.status;
+        r.n_candidates = o.cands;
+        r.n_pairs_refined = o.refined;
+        r.n_scanned = o.scanned;
+        r.n_cells = o.cells;
+        r.n_cand_spheres = o.cand_spheres;
+        r.n_mov = n_mov;
+        r.cyc_scan = o.t_scan - t0;
+        r.cyc_pairs = clock_lo() - o.t_scan;
+        *out = r;
+    }
+    return true;
+}
+
+// One query: warp 0 answers it alone unless it is a large one.
 __global__ void __launch_bounds__(kQueryThreads) k_query(DevBox b, int src, double dx, double dy, double dz,
                                                          double dist, QueryOut *out) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     QuerySmem &sm = *reinterpret_cast<QuerySmem *>(smem_raw);
-    block_query(b, src, Vec3{dx, dy, dz}, dist, sm);
+    __shared__ const int *rec_ptr[REC_INTS];
+    __shared__ int answered;
+    const Vec3 dir{dx, dy, dz};
+    if (threadIdx.x < 32) {
+        if (threadIdx.x == 0) record_rows_init(b, rec_ptr);
+        __syncwarp();
+        using WS = WarpQueryScratch<1024, 1024>;
+        static_assert(sizeof(WS) <= sizeof(QuerySmem), "the scratch stands in the block's plan");
+        const bool ok = warp_query_out(b, b.sc, *reinterpret_cast<WS *>(smem_raw),
+                                       record_rows(b, rec_ptr, threadIdx.x), src, dir, dist, out);
+        if (threadIdx.x == 0) answered = ok;
+    }
+    __syncthreads();
+    if (answered) return;  // block-uniform
+    block_query(b, src, dir, dist, sm);
     if (threadIdx.x == 0) *out = sm.out;
 }
 
@@ -45,6 +94,8 @@ struct QueryIn {
 };
 struct BatchScratch {
     int *next;      // query counter, zero at launch
+    int *n_left;    // queries left to the blocks by k_query_warps, and which
+    int *left;
     size_t stride;  // candidate entries per block (nslots + 1)
     int surv_cap;   // HBM survivors per block
     double *cand_db;
@@ -54,10 +105,39 @@ struct BatchScratch {
     int4 *surv;
     double *surv_res;
 };
-// Threads per query block: 64, 128 or 256 (8, 4 or 2 blocks per SM at 128
-// registers a thread); the first large batch of a box times each and keeps
-// the fastest (results do not depend on it).
-constexpr int kBatchThreadChoices[] = {64, 128, 256};
+// The small queries of a batch, a warp each (taken from a counter); the large
+// ones are listed for k_query_batch, which follows on the stream. A block
+// per query waits for its barriers and for chains of loads that one warp
+// follows as fast; sixteen warps an SM keep as many queries in flight.
+constexpr int kQueryWarps = 4;  // per block
+__global__ void __launch_bounds__(32 * kQueryWarps, 4) k_query_warps(DevBox b, BatchScratch s, int n, int *next,
+                                                                     const QueryIn *in, QueryOut *out) {
+    __shared__ WarpQueryScratch<1024, 4096> scratch[kQueryWarps];
+    __shared__ const int *rec_ptr[REC_INTS];
+    __shared__ DevScalars sc;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (threadIdx.x == 0) {
+        record_rows_init(b, rec_ptr);
+        sc = *b.sc;
+    }
+    __syncthreads();
+    const RecRows rows = record_rows(b, rec_ptr, lane);
+    for (;;) {
+        int q = 0;
+        if (lane == 0) q = atomicAdd(next, 1);
+        q = shfl_i(q, 0);
+        if (q >= n) break;
+        const QueryIn qi = in[q];
+        if (!warp_query_out(b, &sc, scratch[wid], rows, qi.slot, Vec3{qi.dx, qi.dy, qi.dz}, qi.dist, out + q) &&
+            lane == 0)
+            s.left[atomicAdd(s.n_left, 1)] = q;
+        __syncwarp();
+    }
+}
+
+// Large queries, a block each (s.left lists them; all n queries when it is
+// null). 256 threads: what is left here are long pair searches, and the
+// batch ends with the longest.
 template <int NT>
 __global__ void __launch_bounds__(NT, 512 / NT) k_query_batch(DevBox b, BatchScratch s, int n, const QueryIn *in,
                                                               QueryOut *out) {
@@ -75,11 +155,12 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_query_batch(DevBox b, BatchScr
     b.surv = s.surv + size_t(blockIdx.x) * size_t(s.surv_cap);
     b.surv_res = s.surv_res + size_t(blockIdx.x) * size_t(s.surv_cap);
     b.surv_cap = s.surv_cap;
+    if (s.left != nullptr) n = *s.n_left;
     for (;;) {
         if (threadIdx.x == 0) q_cur = atomicAdd(s.next, 1);
         __syncthreads();
-        const int q = q_cur;
-        if (q >= n) break;  // block-uniform
+        if (q_cur >= n) break;  // block-uniform
+        const int q = s.left != nullptr ? s.left[q_cur] : q_cur;
         const QueryIn qi = in[q];
         block_query(b, qi.slot, Vec3{qi.dx, qi.dy, qi.dz}, qi.dist, sm);
         if (threadIdx.x == 0) out[q] = sm.out;
@@ -1325,30 +1406,16 @@ int DeviceBox::query_batch(int n, const int *slots, const double *dirs, const do
                    cuda_ok(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100), err,
                            "cudaFuncSetAttribute");
         };
-        if (!set((const void *)k_query_batch<64>) || !set((const void *)k_query_batch<128>) ||
-            !set((const void *)k_query_batch<256>))
-            return ST_CUDA;
+        if (!set((const void *)k_query_batch<256>)) return ST_CUDA;
         attrs = true;
     }
-    // blocks of each size the GPU holds at once; the scratch is sized for
-    // the most of them
-    auto resident = [&](int nt, int *blocks) {
-        int per_sm = 0;
-        cudaError_t e = nt == 64    ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_query_batch<64>, 64,
-                                                                                    sizeof(QuerySmem))
-                        : nt == 128 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_query_batch<128>, 128,
-                                                                                    sizeof(QuerySmem))
-                                    : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_query_batch<256>, 256,
-                                                                                    sizeof(QuerySmem));
-        *blocks = std::max(1, std::min(n, std::max(1, per_sm) * std::max(1, n_sm)));
-        return cuda_ok(e, err, "occupancy");
-    };
-    int blocks = 1;
-    for (int nt : kBatchThreadChoices) {
-        int nb = 1;
-        if (!resident(nt, &nb)) return ST_CUDA;
-        blocks = std::max(blocks, nb);
-    }
+    constexpr int kThreads = 256;
+    int per_sm = 0;
+    if (!cuda_ok(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_query_batch<kThreads>, kThreads,
+                                                               sizeof(QuerySmem)),
+                 err, "occupancy"))
+        return ST_CUDA;
+    const int blocks = std::max(1, std::min(n, std::max(1, per_sm) * std::max(1, n_sm)));
 
     // scratch layout: counter, inputs, outputs, then per-block candidate and
     // survivor slices
@@ -1362,7 +1429,7 @@ int DeviceBox::query_batch(int n, const int *slots, const double *dirs, const do
         off += (std::max<size_t>(bytes, 16) + 255) & ~size_t(255);
         return at;
     };
-    const size_t o_next = carve(sizeof(int)), o_in = carve(sizeof(QueryIn) * size_t(n)),
+    const size_t o_next = carve(3 * sizeof(int)), o_left = carve(sizeof(int) * size_t(n)), o_in = carve(sizeof(QueryIn) * size_t(n)),
                  o_out = carve(sizeof(QueryOut) * size_t(n)), o_db = carve(8 * ncand), o_key = carve(8 * ncand),
                  o_slot = carve(4 * ncand), o_order = carve(4 * ncand), o_prefix = carve(4 * ncand),
                  o_res = carve(8 * ncand), o_ij = carve(8 * ncand), o_surv = carve(sizeof(int4) * nsurv),
@@ -1378,7 +1445,10 @@ int DeviceBox::query_batch(int n, const int *slots, const double *dirs, const do
         batch_bytes_ = off;
     }
     char *base = static_cast<char *>(batch_mem_);
+    // counters: the blocks' next query, the queries left to them, the warps' next query
     sc.next = reinterpret_cast<int *>(base + o_next);
+    sc.n_left = sc.next + 1;
+    sc.left = reinterpret_cast<int *>(base + o_left);
     sc.cand_db = reinterpret_cast<double *>(base + o_db);
     sc.cand_key = reinterpret_cast<long long *>(base + o_key);
     sc.cand_slot = reinterpret_cast<int *>(base + o_slot);
@@ -1403,45 +1473,27 @@ int DeviceBox::query_batch(int n, const int *slots, const double *dirs, const do
     }
     bool ok = cuda_ok(cudaMemcpyAsync(d_in, hin.data(), sizeof(QueryIn) * size_t(n), cudaMemcpyHostToDevice, s), err,
                       "query upload") &&
-              cuda_ok(cudaMemsetAsync(sc.next, 0, sizeof(int), s), err, "query counter");
-    auto launch = [&](int nt, float *ms) {
-        int nb = 1;
-        if (!resident(nt, &nb)) return false;
-        if (!cuda_ok(cudaMemsetAsync(sc.next, 0, sizeof(int), s), err, "query counter")) return false;
+              cuda_ok(cudaMemsetAsync(sc.next, 0, 3 * sizeof(int), s), err, "query counter");
+    if (ok) {
+        // the small queries by warps, then the rest of them by blocks; calls
+        // of no more queries than blocks the GPU runs at once go to the
+        // blocks at once (a query waits for no other then)
         cudaEventRecord(e0, s);
-        if (nt == 64)
-            k_query_batch<64><<<nb, 64, sizeof(QuerySmem), s>>>(b, sc, n, d_in, d_out);
-        else if (nt == 128)
-            k_query_batch<128><<<nb, 128, sizeof(QuerySmem), s>>>(b, sc, n, d_in, d_out);
-        else
-            k_query_batch<256><<<nb, 256, sizeof(QuerySmem), s>>>(b, sc, n, d_in, d_out);
-        cudaEventRecord(e1, s);
-        if (!cuda_ok(cudaGetLastError(), err, "k_query_batch") || !cuda_ok(cudaEventSynchronize(e1), err, "k_query_batch"))
-            return false;
-        cudaEventElapsedTime(ms, e0, e1);
-        return true;
-    };
-    float ms = 0.f;
-    if (ok && batch_threads_ == 0 && n >= 1024) {
-        // the first large batch: each block size on the same queries (they
-        // only read the box), the fastest kept
-        float best = 0.f;
-        for (int nt : kBatchThreadChoices) {
-            float t = 0.f;
-            ok = ok && launch(nt, &t);
-            if (ok && (best == 0.f || t < best)) {
-                best = t;
-                batch_threads_ = nt;
-            }
+        if (n > blocks) {
+            const int grid = std::min((n + kQueryWarps - 1) / kQueryWarps, 4 * std::max(1, n_sm));
+            k_query_warps<<<grid, 32 * kQueryWarps, 0, s>>>(b, sc, n, sc.next + 2, d_in, d_out);
+        } else {
+            sc.left = nullptr;
         }
-        ms = best;
-    } else if (ok) {
-        ok = launch(batch_threads_ ? batch_threads_ : 256, &ms);
+        k_query_batch<kThreads><<<blocks, kThreads, sizeof(QuerySmem), s>>>(b, sc, n, d_in, d_out);
+        cudaEventRecord(e1, s);
+        ok = cuda_ok(cudaGetLastError(), err, "k_query_batch") &&
+             cuda_ok(cudaMemcpyAsync(hout.data(), d_out, sizeof(QueryOut) * size_t(n), cudaMemcpyDeviceToHost, s), err,
+                     "query download") &&
+             cuda_ok(cudaStreamSynchronize(s), err, "k_query_batch");
     }
-    ok = ok &&
-         cuda_ok(cudaMemcpyAsync(hout.data(), d_out, sizeof(QueryOut) * size_t(n), cudaMemcpyDeviceToHost, s), err,
-                 "query download") &&
-         cuda_ok(cudaStreamSynchronize(s), err, "k_query_batch");
+    float ms = 0.f;
+    if (ok) cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (!ok) return ST_CUDA;

@@ -1041,7 +1041,14 @@ __device__ inline void block_query(const DevBox &b, int src, Vec3 dir, double di
             __syncthreads();
             n_sel = sm.n_sel;
         }
-        for (int f = tid; f < n_other && n_sel > 0; f += NT) {
+        // Fewer candidate spheres than threads: the moving spheres are shared
+        // out among NT / n_other threads each (one thread a candidate sphere
+        // left most of a block idle: 500 moving against 115 candidate spheres
+        // took 315 us on 512 threads).
+        const int parts = n_other < NT ? NT / n_other : 1;
+        const int n_work = n_other * parts;
+        for (int wk = tid; wk < n_work && n_sel > 0; wk += NT) {
+            const int part = wk / n_other, f = wk - part * n_other;
             int lo = 0, hi = nc - 1;
             while (lo < hi) {
                 int mid = (lo + hi + 1) >> 1;
@@ -1076,7 +1083,7 @@ __device__ inline void block_query(const DevBox &b, int src, Vec3 dir, double di
                             for (int x1 = max(0, c1 - 1); x1 <= min(g - 1, c1 + 1); ++x1)
                                 for (int x2 = max(0, c2 - 1); x2 <= min(g - 1, c2 + 1); ++x2) {
                                     const int cell = x1 * g + x2;
-                                    for (int k = sm.cell_prefix[cell]; k < sm.cell_prefix[cell + 1]; ++k) {
+                                    for (int k = sm.cell_prefix[cell] + part; k < sm.cell_prefix[cell + 1]; k += parts) {
                                         const int i = int(sm.mov_sel[k]);
                                         const float4 p = sm.mov[i];
                                         // the shift the capsule test will use for this pair
@@ -1090,7 +1097,8 @@ __device__ inline void block_query(const DevBox &b, int src, Vec3 dir, double di
                                 }
                         }
             } else {
-                for (int ii = 0; ii < n_sel; ++ii) try_pair(t0, (cull && !grid) ? int(sm.mov_sel[ii]) : ii, q, pj, r, jl);
+                for (int ii = part; ii < n_sel; ii += parts)
+                    try_pair(t0, (cull && !grid) ? int(sm.mov_sel[ii]) : ii, q, pj, r, jl);
             }
         }
         __syncthreads();

@@ -21,6 +21,7 @@
 #include "box.cuh"
 #include "merge.cuh"
 #include "rng.hpp"
+#include "warp_query.cuh"
 
 namespace mcacg {
 
@@ -114,30 +115,7 @@ using TreeCacheLarge = TreeCacheT<640>;
 constexpr unsigned long long kTreeHeadroom = 1ULL << 62;
 
 
-// Limits of the steps that one warp runs by itself (step.cuh); what is larger
-// goes to the block.
-constexpr int kWarpCells = 128;   // cells a query visits (four per lane)
-constexpr int kWarpQueue = 256;   // aggregates listed for a query
-constexpr int kWarpCands = 32;    // neighbours past the FP32 screen; sphere pairs to refine
-constexpr int kWarpPairs = 1024;  // sphere pairs screened
-constexpr int kWarpMove = 64;     // spheres translated (no limit where a block is one warp)
-
-// Scratch of a one-warp step.
-struct WarpScratch {
-    int queue[kWarpQueue];
-    // neighbours past the FP32 screen, with their scan keys
-    int scr_slot[kWarpCands];
-    long long scr_key[kWarpCands];
-    // candidates as found, and in filter order (distances as ordered keys)
-    unsigned long long c_db[kWarpCands];
-    long long c_key[kWarpCands];
-    int c_slot[kWarpCands];
-    unsigned long long s_db[kWarpCands];
-    int s_slot[kWarpCands], s_off[kWarpCands], s_pre[kWarpCands];
-    // sphere pairs to refine
-    unsigned long long p_key[kWarpCands], p_ij[kWarpCands];
-    int p_r[kWarpCands], p_si[kWarpCands], p_sj[kWarpCands];
-};
+constexpr int kWarpMove = 64;  // spheres one warp translates (no limit where a block is one warp)
 
 // Scratch of a one-warp merge (at most 32 spheres, 496 pairs). Rows of 33, so
 // that lanes reading one row each meet different banks.
@@ -153,7 +131,7 @@ struct RunSmemT {
     union {
         QS q;
         MS m;
-        WarpScratch w;
+        WarpQueryScratch<256, 1024> w;
         WarpMergeScratch wm;
     } u;
     MergeOut mout;
