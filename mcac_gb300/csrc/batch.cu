@@ -32,8 +32,15 @@ constexpr int kRunThreadChoices[] = {32, 64, 128, 256, 512};
 // an SM (shared memory being the limit there, not registers).
 template <int NT>
 using RunSmemFor = typename std::conditional<(NT <= 32), RunSmemSmall, RunSmem>::type;
+// The device loop's: with 256 threads or more (at most two boxes an SM) a
+// box's steps go in rounds (step.cuh). At four boxes an SM their warps already
+// fill the FP64 pipes that rounds would use: 512 boxes' first 4000 steps, the
+// kernel 98 ms one after another and 106 in rounds of four; rounds win there
+// later in a run only (40 000 steps 785 against 710 ms).
+constexpr int kRoundThreads = 256;
 template <int NT>
-using LoopSmemFor = LoopSmemT<RunSmemFor<NT>>;
+using LoopSmemFor = LoopSmemT<typename std::conditional<(NT >= kRoundThreads), RunSmemRounds, RunSmemFor<NT>>::type,
+                              (NT >= kRoundThreads ? (NT / 32 < kRoundMax ? NT / 32 : kRoundMax) : 1)>;
 // wall time of one launch when boxes run to their stop criteria
 constexpr long long kRunLaunchBudgetNs = 200LL * 1000 * 1000;
 
@@ -76,7 +83,10 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_run(const BoxRun *runs, int n,
     __syncthreads();
     tree_cache_load(R, sm.tree);
     live_load(R, sm.live, sm.u.q.warp_tmp);
-    block_steps(sm, max_steps);
+    if constexpr (LoopSmemFor<NT>::kRounds > 1)
+        block_rounds(sm, max_steps);
+    else
+        block_steps(sm, max_steps);
     __syncthreads();
     {
         const int swords = int(sizeof(RunState) / sizeof(int));

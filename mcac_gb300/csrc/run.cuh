@@ -126,12 +126,20 @@ struct WarpMergeScratch {
     unsigned short pair[496];  // i << 8 | j
 };
 
-template <class QS, class MS, class TC, class LL>
+constexpr int kRoundMax = 7;         // steps of a round at most (step.cuh)
+constexpr int kRoundLook = 16;       // rounds between two looks at their pace
+constexpr int kRoundAlone = 64;      // steps one after another that measure theirs
+constexpr int kRoundAgain = 64;      // looks after which it is measured anew
+constexpr int kRoundBack = 512;      // stretch of steps one after another where those are faster,
+constexpr int kRoundBackMax = 4096;  // doubled up to this
+
+template <class QS, class MS, class TC, class LL, int Rounds>
 struct RunSmemT {
     union {
         QS q;
         MS m;
         WarpQueryScratch<256, 1024> w;
+        WarpQueryScratch<192, 1024> r[Rounds];  // one for each step of a round
         WarpMergeScratch wm;
     } u;
     MergeOut mout;
@@ -157,8 +165,9 @@ struct RunSmemT {
     LL live;                      // the live slots when few are left (box.cuh)
     int split, disappear;         // this step's oxidation events
 };
-using RunSmem = RunSmemT<QuerySmem, MergeSmem, TreeCacheLarge, LiveList>;
-using RunSmemSmall = RunSmemT<QuerySmemSmall, MergeSmemSmall, TreeCache, LiveListNone>;
+using RunSmem = RunSmemT<QuerySmem, MergeSmem, TreeCacheLarge, LiveList, 1>;
+using RunSmemRounds = RunSmemT<QuerySmem, MergeSmem, TreeCacheLarge, LiveList, kRoundMax>;
+using RunSmemSmall = RunSmemT<QuerySmemSmall, MergeSmemSmall, TreeCache, LiveListNone, 1>;
 
 // ------------------------------------------------------------ sum tree
 // Marks the kept levels and copies them (all threads).

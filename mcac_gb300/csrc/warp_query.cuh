@@ -52,8 +52,8 @@ __device__ __forceinline__ double sum3(double v, int g) {
 // holds the two positions' coordinate ax (pa, pb); the direction's are on
 // lanes 0-2 (u). The result is valid on every lane of the group. All lanes
 // of the warp call it.
-__device__ inline double warp_sweep(int g, int ax, double pa, double pb, double r1, double r2, double u, double dist,
-                                    double L) {
+__device__ __forceinline__ double warp_sweep(int g, int ax, double pa, double pb, double r1, double r2, double u,
+                                             double dist, double L) {
     const double dc = r1 + r2;
     const double dc2 = dc * dc;
     const double ua = shfl_d(u, ax), u1 = shfl_d(u, ax == 2 ? 0 : ax + 1), u2 = shfl_d(u, ax == 0 ? 2 : ax - 1);
@@ -269,8 +269,12 @@ __device__ __forceinline__ bool warp_query(const DevBox &b, const DevScalars *sc
     }
     // the listed aggregates: those in the reference's neighbourhood that pass
     // the FP32 screen wait for the FP64 filter, with their scan keys
-    bool found = false;
+    bool found = false, sure = false;
     int n_screen = 0;
+    // the shortened sweep of 'sure': both its reach and its length less by a
+    // margin than the exact ones
+    Sweep32 ws = w;
+    ws.dist = w.dist - margin;
     for (int k0 = 0, cnt = 0; k0 < total; k0 += cnt) {
         cnt = min(32, total - k0);
         const int slot = lane < cnt ? list[k0 + lane] : -1;
@@ -291,6 +295,12 @@ __device__ __forceinline__ bool warp_query(const DevBox &b, const DevScalars *sc
         const bool pass = in && slot != src && capsule_hit(w, of.x, of.y, of.z, rmax_f + of.w + margin);
         const unsigned m = __ballot_sync(all, pass);
         if (n_screen + __popc(m) > kWarpCands) return false;
+        if (m != 0u) {
+            const float inner = rmax_f + of.w - 2.f * margin;
+            sure = __any_sync(all, pass && ws.dist > 0.f && inner > 0.f &&
+                                       w.zmax + 2.f * (rmax_f + of.w + margin) + 8.f * margin < w.L &&
+                                       capsule_hit(ws, of.x, of.y, of.z, inner));
+        }
         if (pass) {
             const int at = n_screen + __popc(m & lanes_below(lane));
             W.scr_slot[at] = slot;
@@ -319,7 +329,18 @@ __device__ __forceinline__ bool warp_query(const DevBox &b, const DevScalars *sc
     const int gi = lane / 3, ax = lane - 3 * gi, g = 3 * gi;
     const double x_g = shfl_d(rec.f, AGG_X + ax);
     int nc = 0;
-    for (int k0 = 0; k0 < n_screen; k0 += 10) {
+    if (n_screen == 1 && sure) {
+        // one neighbour, within reach before the sweep's end by more than the
+        // screen's margins: a candidate without the FP64 sweep, whose value
+        // would only order it among others
+        nc = 1;
+        if (lane == 0) {
+            W.c_db[0] = 0ULL;
+            W.c_key[0] = W.scr_key[0];
+            W.c_slot[0] = W.scr_slot[0];
+        }
+    }
+    for (int k0 = nc > 0 ? n_screen : 0; k0 < n_screen; k0 += 10) {
         const bool act = lane < 30 && k0 + gi < n_screen;
         const int slot = act ? W.scr_slot[k0 + gi] : src;
         const double pb = A(b, AGG_X + ax, slot), r2 = A(b, AGG_RMAX, slot);
@@ -334,6 +355,7 @@ __device__ __forceinline__ bool warp_query(const DevBox &b, const DevScalars *sc
         }
         nc += __popc(m);
     }
+    const bool filtered = !(n_screen == 1 && sure);  // the candidates' d_b are known
     __syncwarp();
     o.cands = nc;
     o.t_scan = clock_lo();
@@ -419,8 +441,18 @@ __device__ __forceinline__ bool warp_query(const DevBox &b, const DevScalars *sc
         const bool act = lane < 30 && k0 + gi < n_hit;
         const int k = act ? k0 + gi : 0;
         const int si = W.p_si[k], sj = W.p_sj[k];
-        const double res = warp_sweep(g, ax, S(b, SPH_X + ax, si), S(b, SPH_X + ax, sj), S(b, SPH_R, si),
-                                      S(b, SPH_R, sj), dl, full, b.L);
+        const double xi = S(b, SPH_X + ax, si), xj = S(b, SPH_X + ax, sj), ri = S(b, SPH_R, si), rj = S(b, SPH_R, sj);
+        // two single spheres at their aggregates' centres: the filter's sweep
+        // was this one
+        const int oslot = W.s_slot[W.p_r[k]];
+        const bool same = filtered && ((dbits(xi) ^ dbits(x_g)) | (dbits(ri) ^ dbits(rmax)) |
+                                       (dbits(xj) ^ dbits(A(b, AGG_X + ax, oslot))) |
+                                       (dbits(rj) ^ dbits(A(b, AGG_RMAX, oslot)))) == 0;
+        double res;
+        if (__all_sync(all, same || !act))
+            res = dkey_inv(W.s_db[W.p_r[k]]);
+        else
+            res = warp_sweep(g, ax, xi, xj, ri, rj, dl, full, b.L);
         if (act && ax == 0) W.p_key[k] = res < CUDART_INF ? dkey(res) : ~0ULL;
     }
     __syncwarp();
