@@ -9,6 +9,13 @@
 // first warp, in step (any block size of 32 threads or more works). The
 // O(n^2) intra-aggregate contact search is screened in FP32 and refined in
 // FP64; its pairs are put back in (i, j) order before they are summed.
+//
+// What bounds it: the two rounds of ordered sums, 64 cycles a term (an FP64
+// addition after another), with the terms' loads eight ahead of them. The
+// screen's survivors are listed first and refined together, a pair on each
+// thread: refined where they were found they came one or two a warp at a time,
+// each some 50 FP64 instructions on all 32 lanes' time, the larger part of a
+// merge.
 #pragma once
 #include "box.cuh"
 
@@ -25,9 +32,10 @@ struct MergeSmemT {
     double r_cm[3];
     double sums[kSumSeries];
     double vol_raw, overlap, coord;
+    double fin[5];  // the position, mean diameter and mean sphere volume
     float ext, rmax_f;  // bound of |relative position| + r, largest radius (FP32)
     double rmax_warp[32];
-    float tile_f[kPairTile * 4];
+    alignas(16) float4 tile_f[kPairTile];
     int warp_tmp[32];
     float warp_f[32];
     int keep, removed, mysph, othsph;
@@ -109,9 +117,26 @@ static __device__ __noinline__ void block_compact_pool(const DevBox &b, int *war
 }
 
 // Sequential (list-order) sum of one work series, as the reference's loops.
+// The terms are loaded eight ahead of the addition (512 cycles, more than the
+// loads take).
 __device__ __forceinline__ double ordered_sum(const double *v, int n) {
-    double acc = 0.0;
-    for (int i = 0; i < n; ++i) acc = acc + v[i];
+    double acc = 0.0, t[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) t[u] = u < n ? v[u] : 0.0;
+    int i = 0;
+#pragma unroll 1
+    for (; i + 8 <= n; i += 8) {
+        double next[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) next[u] = i + 8 + u < n ? v[i + 8 + u] : 0.0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) acc = acc + t[u];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) t[u] = next[u];
+    }
+#pragma unroll
+    for (int u = 0; u < 7; ++u)
+        if (i + u < n) acc = acc + t[u];
     return acc;
 }
 
@@ -227,24 +252,17 @@ __device__ inline void block_pair_scan(const DevBox &b, const int *mem, int n, S
         }
         __syncthreads();
     } else {
+    const int parts = n < NT ? NT / n : 1, rows = NT / parts;
     for (int j0 = 0; j0 < n; j0 += kPairTile) {
         const int nt = min(kPairTile, n - j0);
-        for (int k = tid; k < nt; k += NT) {
-            float4 v = relf[j0 + k];
-            sm.tile_f[4 * k + 0] = v.x;
-            sm.tile_f[4 * k + 1] = v.y;
-            sm.tile_f[4 * k + 2] = v.z;
-            sm.tile_f[4 * k + 3] = v.w;
-        }
+        for (int k = tid; k < nt; k += NT) sm.tile_f[k] = relf[j0 + k];
         __syncthreads();
-        for (int i = tid; i < min(n, j0 + nt); i += NT) {
+        // fewer spheres than threads: 'parts' threads share a sphere's row
+        // (a last thread beyond the shares starts at a row past n)
+        for (int i = tid / parts; i < min(n, j0 + nt); i += rows) {
             const float4 pi_ = relf[i];
-            int jstart = max(i + 1, j0) - j0;
-            for (int jj = jstart; jj < nt; ++jj) {
-                const float4 pj_ = make_float4(sm.tile_f[4 * jj + 0], sm.tile_f[4 * jj + 1], sm.tile_f[4 * jj + 2],
-                                               sm.tile_f[4 * jj + 3]);
-                pair_test(i, j0 + jj, pi_, pj_);
-            }
+            for (int jj = max(i + 1, j0) - j0 + tid % parts; jj < nt; jj += parts)
+                pair_test(i, j0 + jj, pi_, sm.tile_f[jj]);
         }
         __syncthreads();
     }
@@ -403,28 +421,39 @@ __device__ inline void block_merge(const DevBox &b, int ms, int os, int mslot, i
     __syncthreads();
     const int *mem = pool_id + new_off;
 
-    // ---- update_distances_and_overlapping: contact pairs i < j
-    for (int k = tid; k <= n; k += NT) b.row_cnt[k] = 0;
-    if (tid == 0) b.counters[0] = 0;
-    block_pair_scan(b, mem, n, sm, 0.f, [&](int i, int j) {
+    // ---- update_distances_and_overlapping: contact pairs i < j. The screen's
+    // survivors are listed, then tested; a list that does not fit is built
+    // again from the tested ones only.
+    const double contact = 1. + kCoordinationEpsilon;
+    auto pair_distance = [&](int i, int j, double *rsum) {
         const int si = mem[i], sj = mem[j];
-        double ex = S(b, SPH_RX, si) - S(b, SPH_RX, sj);
-        double ey = S(b, SPH_RY, si) - S(b, SPH_RY, sj);
-        double ez = S(b, SPH_RZ, si) - S(b, SPH_RZ, sj);
-        double dist = sqrt(ex * ex + ey * ey + ez * ez);
-        double rsum = S(b, SPH_R, si) + S(b, SPH_R, sj);
-        if (dist <= (1. + kCoordinationEpsilon) * rsum) {
-            int p = atomicAdd(&b.counters[0], 1);
+        const double ex = S(b, SPH_RX, si) - S(b, SPH_RX, sj);
+        const double ey = S(b, SPH_RY, si) - S(b, SPH_RY, sj);
+        const double ez = S(b, SPH_RZ, si) - S(b, SPH_RZ, sj);
+        *rsum = S(b, SPH_R, si) + S(b, SPH_R, sj);
+        return sqrt(ex * ex + ey * ey + ez * ez);
+    };
+    int listed = 0, P = 0;
+    for (int tested = 0; tested < 2; ++tested) {
+        for (int k = tid; k <= n; k += NT) b.row_cnt[k] = 0;
+        if (tid == 0) {
+            b.counters[0] = 0;
+            sm.n_pairs = 0;
+        }
+        block_pair_scan(b, mem, n, sm, 0.f, [&](int i, int j) {
+            double rsum = 0.0;
+            if (tested && !(pair_distance(i, j, &rsum) <= contact * rsum)) return;
+            const int p = atomicAdd(&b.counters[0], 1);
             if (p < b.pair_cap) {
                 b.pair_tmp_i[p] = i;
                 b.pair_tmp_j[p] = j;
-                b.pair_tmp_d[p] = dist;
-                atomicAdd(&b.row_cnt[i], 1);
             }
-        }
-    });
-    const int P = b.counters[0];
-    if (P > b.pair_cap) {
+        });
+        listed = b.counters[0];  // block-uniform: the scan ends on a barrier
+        if (listed <= b.pair_cap) break;
+        __syncthreads();
+    }
+    if (listed > b.pair_cap) {
         if (tid == 0) {
             sc->status = ST_CAPACITY;
             out->merged = 1;
@@ -433,10 +462,25 @@ __device__ inline void block_merge(const DevBox &b, int ms, int os, int mslot, i
         __syncthreads();
         return;
     }
+    for (int p = tid; p < listed; p += NT) {
+        const int i = b.pair_tmp_i[p];
+        double rsum;
+        const double dist = pair_distance(i, b.pair_tmp_j[p], &rsum);
+        if (dist <= contact * rsum) {
+            b.pair_tmp_d[p] = dist;
+            atomicAdd(&b.row_cnt[i], 1);
+            atomicAdd(&sm.n_pairs, 1);
+        } else {
+            b.pair_tmp_i[p] = -1;
+        }
+    }
+    __syncthreads();
+    P = sm.n_pairs;
     // counting sort of the pairs by i, then by j within a row
     block_scan_global(b.row_cnt, n + 1, sm.warp_tmp);
-    for (int p = tid; p < P; p += NT) {
+    for (int p = tid; p < listed; p += NT) {
         int i = b.pair_tmp_i[p];
+        if (i < 0) continue;
         int dst = atomicAdd(&b.row_cnt[i], 1);
         b.pair_i[dst] = i;
         b.pair_j[dst] = b.pair_tmp_j[p];
@@ -487,13 +531,13 @@ __device__ inline void block_merge(const DevBox &b, int ms, int os, int mslot, i
         b.sph_volw[s] = vol;
     }
     __syncthreads();
-    // overlapping's terms (rsum - d) / rsum of the (i, j)-ordered pairs, formed
-    // in parallel (each one rounding as in the reference); summed in pair
-    // order below. The pair sort's scratch is free by now.
+    // overlapping's terms 2 (rsum - d) / rsum of the (i, j)-ordered pairs, formed
+    // in parallel (each one rounding as in the reference, the doubling exact);
+    // summed in pair order below. The pair sort's scratch is free by now.
     double *ov_terms = b.pair_tmp_d;
     for (int p = tid; p < P; p += NT) {
         const double rsum = S(b, SPH_R, mem[b.pair_i[p]]) + S(b, SPH_R, mem[b.pair_j[p]]);
-        ov_terms[p] = (rsum - b.pair_d[p]) / rsum;
+        ov_terms[p] = 2.0 * ((rsum - b.pair_d[p]) / rsum);
     }
     __syncthreads();
     {
@@ -501,12 +545,7 @@ __device__ inline void block_merge(const DevBox &b, int ms, int os, int mslot, i
         if (tid < 7) sm.sums[tid] = ordered_sum(wv + size_t(tid) * W, n);
         // the overlap sum, sequential over the pairs, on the second warp
         // when there is one (beside the seven)
-        if (tid == (NT > 32 ? 32 : 0)) {
-            double ov = 0.0;
-            for (int p = 0; p < P; ++p) ov += 2.0 * ov_terms[p];
-            sm.sums[7] = ov;
-            sm.n_pairs = P;
-        }
+        if (tid == (NT > 32 ? 32 : 0)) sm.sums[7] = ordered_sum(ov_terms, P);
     }
     __syncthreads();
     if (tid == 0) {
@@ -528,13 +567,8 @@ __device__ inline void block_merge(const DevBox &b, int ms, int os, int mslot, i
     }
     __syncthreads();
     const double V = sm.sums[0], Sf = sm.sums[1];
-    if (tid == 0) {
-        if (V <= 0 || Sf <= 0) sm.status = ST_VOL_SURF;
-        double cx = sm.sums[2] / V, cy = sm.sums[3] / V, cz = sm.sums[4] / V;
-        sm.r_cm[0] = cx;
-        sm.r_cm[1] = cy;
-        sm.r_cm[2] = cz;
-    }
+    if (tid == 0 && (V <= 0 || Sf <= 0)) sm.status = ST_VOL_SURF;
+    if (tid < 3) sm.r_cm[tid] = sm.sums[2 + tid] / V;
     __syncthreads();
     if (sm.status != ST_OK) {
         if (tid == 0) {
@@ -568,33 +602,29 @@ __device__ inline void block_merge(const DevBox &b, int ms, int os, int mslot, i
         cell_remove(b, cell_index(b, b.agg_cell[removed]), removed);
         if (b.fine_div > 0) fine_unlink(b, removed);
     }
-    double x = 0.0, y = 0.0, z = 0.0, rmax = 0.0, vol_pp = 0.0;
+    // the aggregate's position, an axis on each of threads 0-2; its mean
+    // diameter and mean sphere volume on threads 3 and 4
+    if (tid < 5) {
+        const double q = (tid == 3 ? 2 * sm.sums[6] : (tid == 4 ? sm.vol_raw : 0.0)) / static_cast<double>(n);
+        const double x = tid < 3 ? periodic_position(S(b, SPH_X + tid, mem[0]) + sm.r_cm[tid], b.L) : q;
+        sm.fin[tid] = x;
+        if (tid < 4) A(b, tid < 3 ? AGG_X + tid : AGG_DP, keep) = x;
+        if (tid < 3) A(b, AGG_RX + tid, keep) = sm.r_cm[tid];
+    }
+    if (tid < 32) __syncwarp();
     if (tid == 0) {
+        double rmax = 0.0;
         for (int k = 0; k < NT / 32; ++k) rmax = dmax(rmax, sm.rmax_warp[k]);
-        double arg = ordered_sum(wv + 7 * W, n);
-        double brg = sm.sums[5];
-        double rg = sqrt(fabs((arg + (3. / 5.) * brg) / V));
-        double dp = 2 * sm.sums[6] / static_cast<double>(n);
-        vol_pp = sm.vol_raw / static_cast<double>(n);
-        const double overlapping = sm.overlap, coordination = sm.coord;
-        const int s0 = mem[0];
-        x = periodic_position(S(b, SPH_X, s0) + sm.r_cm[0], b.L);
-        y = periodic_position(S(b, SPH_Y, s0) + sm.r_cm[1], b.L);
-        z = periodic_position(S(b, SPH_Z, s0) + sm.r_cm[2], b.L);
-        A(b, AGG_RG, keep) = rg;
+        const double arg = ordered_sum(wv + 7 * W, n);
+        const double brg = sm.sums[5];
+        A(b, AGG_RG, keep) = sqrt(fabs((arg + (3. / 5.) * brg) / V));
         A(b, AGG_RMAX, keep) = rmax;
         A(b, AGG_VOLUME, keep) = V;
         A(b, AGG_SURFACE, keep) = Sf;
-        A(b, AGG_X, keep) = x;
-        A(b, AGG_Y, keep) = y;
-        A(b, AGG_Z, keep) = z;
-        A(b, AGG_RX, keep) = sm.r_cm[0];
-        A(b, AGG_RY, keep) = sm.r_cm[1];
-        A(b, AGG_RZ, keep) = sm.r_cm[2];
-        A(b, AGG_DP, keep) = dp;
-        A(b, AGG_OVERLAPPING, keep) = overlapping;
-        A(b, AGG_COORDINATION_NUMBER, keep) = coordination;
-        b.agg_f4[keep] = make_float4(float(x), float(y), float(z), float(rmax));
+        A(b, AGG_OVERLAPPING, keep) = sm.overlap;
+        A(b, AGG_COORDINATION_NUMBER, keep) = sm.coord;
+        b.agg_f4[keep] = make_float4(float(sm.fin[0]), float(sm.fin[1]), float(sm.fin[2]), float(rmax));
+        if (rmax > sc->maxradius) sc->maxradius = rmax;
     }
     __syncthreads();
     if (tid == 0) {
@@ -602,18 +632,17 @@ __device__ inline void block_merge(const DevBox &b, int ms, int os, int mslot, i
             cell_remove(b, cell_index(b, b.agg_cell[removed]), removed);
             if (b.fine_div > 0) fine_unlink(b, removed);
         }
-        regrid(b, keep, Vec3{x, y, z});
-        if (rmax > sc->maxradius) sc->maxradius = rmax;
+        regrid(b, keep, Vec3{sm.fin[0], sm.fin[1], sm.fin[2]});
         out->merged = 1;
         out->status = ST_OK;
         out->keep = keep;
         out->removed = removed;
         out->n = n;
         out->n_pairs = P;
-        for (int f = 0; f < AGG_NFIELDS; ++f) out->fields[f] = A(b, f, keep);
-        out->vol_pp = vol_pp;
+        out->vol_pp = sm.fin[4];
         out->maxradius = sc->maxradius;
     }
+    for (int f = tid; f < AGG_NFIELDS; f += NT) out->fields[f] = A(b, f, keep);
     __syncthreads();
 }
 
