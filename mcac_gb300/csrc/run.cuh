@@ -301,6 +301,35 @@ __device__ inline unsigned long long tree_set(const BoxRun &R, TC &c, int slot, 
     return total;
 }
 
+// Warp 0: the tree after a merge, a level on each lane (the leaves' changes
+// carry over to every ancestor by themselves, exactly): 'removed' gives up
+// its weight, 'keep' takes the weight wk. Returns the new total.
+template <class TC>
+__device__ __forceinline__ unsigned long long tree_merge(const BoxRun &R, TC &c, unsigned long long total, int keep,
+                                                         int removed, unsigned long long w_keep,
+                                                         unsigned long long w_removed, unsigned long long wk) {
+    const int lane = threadIdx.x & 31;
+    if (lane < R.tree_levels) {
+        const int sh = 5 * lane, gk = keep >> sh, gr = removed >> sh, co = c.coff[lane];
+        unsigned long long *lev = R.tree + R.tree_off[lane];
+        unsigned long long *own = c.v + (co >= 0 ? co : 0);
+        unsigned long long vr = 0ULL, vk = wk;
+        if (lane > 0) {
+            vr = co >= 0 ? own[gr] : lev[gr];
+            vk = gk == gr ? vr : (co >= 0 ? own[gk] : lev[gk]);
+            vr -= w_removed;
+            vk = (gk == gr ? vr : vk) - w_keep + wk;
+        }
+        if (gk != gr) {
+            lev[gr] = vr;
+            if (co >= 0) own[gr] = vr;
+        }
+        lev[gk] = vk;
+        if (co >= 0) own[gk] = vk;
+    }
+    return total - w_keep - w_removed + wk;
+}
+
 // The loop state's FP64 total weight and its inverse (the time increment of
 // a step) from the tree's integer total.
 __device__ __forceinline__ void tree_total_to_state(RunState &st, unsigned long long total) {
@@ -1630,9 +1659,11 @@ __device__ inline void commit_merge(const BoxRun &R, RS &sm) {
     __syncthreads();
     if (sm.stop || !sm.merged || R.phys.growth) return;
     if (tid < 32) {
-        tree_set(R, sm.tree, sm.removed, 0ULL);
+        const unsigned long long *leaves = R.tree + R.tree_off[0];
+        const unsigned long long w_keep = leaves[sm.keep], w_removed = leaves[sm.removed];
         const unsigned long long wk = tree_weight(st, A(b, AGG_TIME_STEP, sm.keep));
-        const unsigned long long total = tree_set(R, sm.tree, sm.keep, wk);
+        const unsigned long long total =
+            tree_merge(R, sm.tree, st.tree_total, sm.keep, sm.removed, w_keep, w_removed, wk);
         if (tid == 0) {
             tree_total_to_state(st, total);
             sm.rescale = total > kTreeHeadroom;  // a new scale keeps the total clear of 2^64

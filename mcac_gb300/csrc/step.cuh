@@ -419,25 +419,7 @@ __device__ __noinline__ int warp_merge() {
         st.c_merged_spheres += n;
         st.c_merge_pairs += Pc;
     }
-    // the pick tree, a level on each lane
-    if (lane < R.tree_levels) {
-        const int sh = 5 * lane, gk = keep >> sh, gr = removed >> sh, co = sm.tree.coff[lane];
-        unsigned long long *lev = R.tree + R.tree_off[lane];
-        unsigned long long *own = sm.tree.v + (co >= 0 ? co : 0);
-        unsigned long long vr = 0ULL, vk = wk;
-        if (lane > 0) {
-            vr = co >= 0 ? own[gr] : lev[gr];
-            vk = gk == gr ? vr : (co >= 0 ? own[gk] : lev[gk]);
-            vr -= w_removed;
-            vk = (gk == gr ? vr : vk) - w_keep + wk;
-        }
-        if (gk != gr) {
-            lev[gr] = vr;
-            if (co >= 0) own[gr] = vr;
-        }
-        lev[gk] = vk;
-        if (co >= 0) own[gk] = vk;
-    }
+    tree_merge(R, sm.tree, 0ULL, keep, removed, w_keep, w_removed, wk);
     const bool rescale = total > kTreeHeadroom;  // a new scale keeps the total clear of 2^64
     if (lane == 0) tree_total_to_state(st, total);
     if (sm.live.on) warp_live_merge(sm.live, keep, removed, wk);
@@ -1126,12 +1108,12 @@ __device__ inline void block_rounds(LS &sm, long long max_steps) {
                 }
                 if (st.finished || st.status != ST_OK || sm.stop) k = 0;
                 if (k > 0 && sm.deadline != 0ULL && global_ns() >= sm.deadline) k = 0;
-                sm.n_jobs = k;
+                sm.n_jobs = k > 0 && sm.seq > 0 ? -1 : k;  // -1: warp 0 alone
             }
             __syncthreads();
             jobs = sm.n_jobs;
-            if (jobs <= 0) return;  // block-uniform
-            alone = sm.seq > 0;
+            if (jobs == 0) return;  // block-uniform
+            alone = jobs < 0;
             if (alone) jobs = 1;
         } else if (wid == 0) {  // a step goes on after the block's operation, and the next may follow
             const int op = warp_steps_call<LS>(phase, t_phase);
@@ -1297,6 +1279,7 @@ __device__ inline void block_rounds(LS &sm, long long max_steps) {
                 const bool over = go != STEP_NEXT || finished || seq <= 0 || n_done >= quota ||
                                   (sm.deadline != 0ULL && __shfl_sync(0xffffffffu, int(global_ns() >= sm.deadline), 0));
                 if (over) {
+                    __syncwarp();
                     if (lane == 0) {
                         sm.left -= n_done;
                         sm.seq = R.phys.growth ? INT_MAX : seq;
