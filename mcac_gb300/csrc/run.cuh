@@ -1296,7 +1296,11 @@ __device__ inline void block_split_slot(const BoxRun &R, RS &sm, int a) {
     for (int p = tid; p < P; p += NT)
         if (!uf_unite(parent, b.pair_tmp_i[p], b.pair_tmp_j[p], n)) b.counters[4] = 1;
     __syncthreads();
-    for (int i = tid; i < n; i += NT) parent[i] = uf_find(parent, i);
+    // each sphere's root, in an array of its own: stored into the forest, a
+    // root could be overwritten by the path halving of a walk under way with
+    // an ancestor that is not a root (and the sphere be given a wrong part)
+    int *root = b.pair_tmp_i;  // the contacts are done with
+    for (int i = tid; i < n; i += NT) root[i] = uf_find(parent, i);
     __syncthreads();
     if (b.counters[4] != 0) {
         if (tid == 0) sc->status = ST_UNKNOWN;
@@ -1305,7 +1309,7 @@ __device__ inline void block_split_slot(const BoxRun &R, RS &sm, int a) {
     }
     // parts in the order of their first sphere
     int *rank = reinterpret_cast<int *>(b.work);  // n + 1
-    for (int i = tid; i < n; i += NT) rank[i] = parent[i] == i ? 1 : 0;
+    for (int i = tid; i < n; i += NT) rank[i] = root[i] == i ? 1 : 0;
     __syncthreads();
     const int K = block_scan_global(rank, n, sm.u.m.warp_tmp);
     if (K < 2) return;
@@ -1316,7 +1320,7 @@ __device__ inline void block_split_slot(const BoxRun &R, RS &sm, int a) {
     for (int c = tid; c <= K; c += NT) cnt[c] = 0;
     __syncthreads();
     for (int i = tid; i < n; i += NT) {
-        const int c = rank[parent[i]];
+        const int c = rank[root[i]];
         part[i] = c;
         atomicAdd(&cnt[c], 1);
     }
