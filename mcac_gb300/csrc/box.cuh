@@ -234,16 +234,42 @@ __device__ __forceinline__ double dkey_inv(unsigned long long k) {
 // 560 for a division, 690 for a square root after an add). The helpers below
 // compare doubles as integers, which gives the same answers.
 __device__ __forceinline__ long long dbits(double v) { return __double_as_longlong(v); }
-// |a| < b for b > 0 (false for NaN)
+constexpr unsigned long long kInfBits = 0x7ff0000000000000ULL;
+__device__ __forceinline__ bool is_nan(double v) { return ((unsigned long long)dbits(v) << 1) > (kInfBits << 1); }
+// |a| < b for b > 0 (false for a NaN)
 __device__ __forceinline__ bool abs_lt(double a, double b) {
     return (dbits(a) & 0x7fffffffffffffffLL) < dbits(b);
 }
-// a <= b for non-negative a and b (a NaN compares as larger)
-__device__ __forceinline__ bool nonneg_le(double a, double b) { return dbits(a) <= dbits(b); }
+// a <= b for non-negative a (false for a NaN of either sign on either side, and
+// for a negative b): a NaN made by the GPU has the sign bit set, so compared
+// as a signed integer it would be below every number
+__device__ __forceinline__ bool nonneg_le(double a, double b) {
+    const unsigned long long ub = dbits(b);
+    return (unsigned long long)dbits(a) <= ub && ub <= kInfBits;
+}
+// max(a, b) of a non-negative a, and of b where it is a positive number (a NaN
+// and a negative b are left out, as by dmax)
+__device__ __forceinline__ long long nonneg_max_bits(long long a, long long b) {
+    return a < b && b <= (long long)kInfBits ? b : a;
+}
+__device__ __forceinline__ double nonneg_max(double a, double b) {
+    return __longlong_as_double(nonneg_max_bits(dbits(a), dbits(b)));
+}
+// a <= 0 (false for NaN)
+__device__ __forceinline__ bool not_positive(double a) { return dbits(a) == 0 || (dbits(a) < 0 && !is_nan(a)); }
+// a > 0, normal, and 2 a finite
+__device__ __forceinline__ bool positive_normal(double a) {
+    return (unsigned long long)dbits(a) - (1ULL << 52) < kInfBits - (2ULL << 52);
+}
 // a < 0 (false for -0)
 __device__ __forceinline__ bool neg(double a) { return dbits(a) < 0 && dbits(a) != LLONG_MIN; }
 // 0.5 * x by its exponent, for normal x whose half is normal
 __device__ __forceinline__ double half_of(double x) { return __longlong_as_double(dbits(x) - (1LL << 52)); }
+static __device__ __noinline__ double fp64_half(double x) { return 0.5 * x; }
+// 0.5 * x for any x
+__device__ __forceinline__ double half_any(double x) {
+    return positive_normal(x) && dbits(x) >= (2LL << 52) ? half_of(x) : fp64_half(x);
+}
 static __device__ __noinline__ double periodic_distance_call(double d, double L) { return periodic_distance(d, L); }
 // periodic_distance: the wrap loops only run for |d| >= L/2
 __device__ __forceinline__ double wrap_distance(double d, double L) {

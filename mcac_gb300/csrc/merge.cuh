@@ -118,9 +118,6 @@ static __device__ __noinline__ void block_compact_pool(const DevBox &b, int *war
     __syncthreads();
 }
 
-// dmax of two values that are 0 or positive (their bits order them)
-__device__ __forceinline__ double nonneg_max(double a, double b) { return dbits(a) < dbits(b) ? b : a; }
-
 // Sequential (list-order) sum of one work series, as the reference's loops.
 // The terms are loaded eight ahead of the addition (512 cycles, more than the
 // loads take).

@@ -651,7 +651,9 @@ __device__ inline bool thread_update_monomer(const DevBox &b, int a, bool full, 
     const double volw = full ? vol : b.sph_volw[s], volume = full ? vol : A(b, AGG_VOLUME, a);
     const long long L = dbits(b.L);
     if ((dbits(rel) | dbits(rely) | dbits(relz)) != 0) return false;
-    if (dbits(r) <= 0 || dbits(vol) <= 0 || dbits(sur) <= 0 || dbits(volw) <= 0 || dbits(volume) <= 0) return false;
+    if (!(positive_normal(r) && positive_normal(vol) && positive_normal(sur) && positive_normal(volw) &&
+          positive_normal(volume)))
+        return false;
     if (dbits(x) < 0 || dbits(x) >= L || dbits(y) < 0 || dbits(y) >= L || dbits(z) < 0 || dbits(z) >= L) return false;
     if (full) {
         b.sph_volw[s] = vol;
@@ -823,8 +825,7 @@ static __device__ __noinline__ double warp_update_geometry(const DevBox &b, int 
             const int cnt = min(32, n - k0);
             const double dx = x - rx, dy = y - ry, dz = z - rz;
             const double dc = fp64_sqrt(dx * dx + dy * dy + dz * dz);
-            const long long far = lane < cnt ? dbits(r + dc) : 0;  // below zero (an empty sphere): not taken
-            rmax_bits = far > rmax_bits ? far : rmax_bits;
+            if (lane < cnt) rmax_bits = nonneg_max_bits(rmax_bits, dbits(r + dc));
             W.term[0][lane] = volw * (dc * dc);
             __syncwarp();
             fetch(k0 + 32 + lane);
@@ -876,8 +877,8 @@ __device__ inline double warp_update_aggregate(const BoxRun &R, int a, bool full
     double vol_pp = 0.0;
     const double rmax = warp_update_geometry(b, a, full, W, &vol_pp);
     const double dp = A(b, AGG_DP, a);
-    const float4 v = physics_f32(R.phys, float(half_of(dp)), float(A(b, AGG_VOLUME, a)), float(vol_pp));
-    const double dgdp = fp64_div(A(b, AGG_RG, a), half_of(dp));
+    const float4 v = physics_f32(R.phys, float(half_any(dp)), float(A(b, AGG_VOLUME, a)), float(vol_pp));
+    const double dgdp = fp64_div(A(b, AGG_RG, a), half_any(dp));
     if ((threadIdx.x & 31) == 0) {
         A(b, AGG_F_AGG, a) = double(v.x);
         A(b, AGG_D_M, a) = double(v.y);
@@ -1012,7 +1013,7 @@ __device__ inline void block_update_all(const BoxRun &R, RS &sm, bool full) {
         UpdScratch &W = reinterpret_cast<UpdScratch *>(&sm.u)[wid];
         for (int k = next(&sm.next_large, 1); k < sm.n_listed; k = next(&sm.next_large, 1)) {
             const double rm = warp_update_aggregate(R, list[k], full, W);
-            rmax_d = dbits(rm) > dbits(rmax_d) ? rm : rmax_d;
+            rmax_d = nonneg_max(rmax_d, rm);
             if (lane == 0) note_cell(list[k]);
         }
     }
@@ -1020,7 +1021,7 @@ __device__ inline void block_update_all(const BoxRun &R, RS &sm, bool full) {
         if (k + lane >= sm.n_small) continue;
         const int a = small[k + lane];
         const double rm = thread_update_aggregate(R, a, full);
-        rmax_d = dbits(rm) > dbits(rmax_d) ? rm : rmax_d;
+        rmax_d = nonneg_max(rmax_d, rm);
         note_cell(a);
     }
     __syncwarp();
@@ -1048,7 +1049,7 @@ __device__ inline void block_update_all(const BoxRun &R, RS &sm, bool full) {
             rm = thread_update_aggregate(R, a, full);
             note_cell(a);
         }
-        rmax_d = dbits(rm) > dbits(rmax_d) ? rm : rmax_d;
+        rmax_d = nonneg_max(rmax_d, rm);
     }
     __syncwarp();
     // block max of r_max (bits of a non-negative double order like integers)

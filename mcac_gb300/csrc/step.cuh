@@ -210,7 +210,8 @@ __device__ __noinline__ int warp_merge() {
         const double d = wrap_distance(pm - po, b.L);
         const double d2 = sum3(d * d, 0);
         const double s = rms + ros;
-        if (!(dkey(d2 - s * s) <= dkey(kContactEpsilon))) return WM_DONE;  // the spheres no longer touch
+        const double gap = d2 - s * s;
+        if (!(dkey(gap) <= dkey(kContactEpsilon)) || is_nan(gap)) return WM_DONE;  // the spheres no longer touch
     }
     const double diff = (rel_my + wrap_distance(my == ms ? po - pm : pm - po, b.L)) - rel_oth;
     // round 2: the members, and the removed slot's cell
@@ -341,7 +342,7 @@ __device__ __noinline__ int warp_merge() {
         for (int k = 0; k < most; ++k) acc = acc + (k < lim ? v[k] : 0.0);
     }
     const double V = shfl_d(acc, 0), Sf = shfl_d(acc, 1);
-    if (dbits(V) <= 0 || dbits(Sf) <= 0) {
+    if (not_positive(V) || not_positive(Sf)) {
         if (lane == 0) {
             sc->status = ST_VOL_SURF;
             st.status = ST_VOL_SURF;
@@ -354,7 +355,7 @@ __device__ __noinline__ int warp_merge() {
     const double cx = shfl_d(cm, 2), cy = shfl_d(cm, 3), cz = shfl_d(cm, 4);
     const double dx = rx - cx, dy = ry - cy, dz = rz - cz;
     const double dcen = fp64_sqrt(dx * dx + dy * dy + dz * dz);
-    long long rmax_bits = act ? dbits(r + dcen) : 0;  // non-negative: integer order
+    long long rmax_bits = act ? nonneg_max_bits(0, dbits(r + dcen)) : 0;  // non-negative: integer order
     M.term[7][lane] = vol * (dcen * dcen);
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) {
@@ -378,11 +379,11 @@ __device__ __noinline__ int warp_merge() {
     const double dp = shfl_d(quo, 1), vol_pp = shfl_d(quo, 2);
     const double overlapping = Pc > 0 ? shfl_d(quo, 3) : 0.0, coordination = Pc > 0 ? shfl_d(quo, 4) : 0.0;
     const double x = wrap_position(ref + shfl_d(cm, 2 + a3), b.L);  // lanes 0-2
-    const float cf = float(lane < 3 ? x : (lane == 3 ? rmax : (lane == 4 ? V : (lane == 5 ? vol_pp : half_of(dp)))));
+    const float cf = float(lane < 3 ? x : (lane == 3 ? rmax : (lane == 4 ? V : (lane == 5 ? vol_pp : half_any(dp)))));
     const float4 ph = physics_f32(R.phys, shfl_f(cf, 6), shfl_f(cf, 4), shfl_f(cf, 5));
     const double phd = double(lane == 0 ? ph.x : (lane == 1 ? ph.y : (lane == 2 ? ph.z : ph.w)));
     // lane 0: Rg / (dp / 2), lane 2: 1 / time step
-    const double rec = fp64_div(lane == 0 ? rg : 1.0, lane == 0 ? half_of(dp) : phd);
+    const double rec = fp64_div(lane == 0 ? rg : 1.0, lane == 0 ? half_any(dp) : phd);
     unsigned long long wk = __double2ull_rn(fmin(rec * st.tree_scale, double(kTreeHeadroom)));
     wk = __shfl_sync(all, wk > 0ULL ? wk : 1ULL, 2);
     const double time = (shfl_d(rk.f, AGG_TIME) + shfl_d(rr.f, AGG_TIME)) - st.time;
@@ -414,7 +415,7 @@ __device__ __noinline__ int warp_merge() {
         A(b, AGG_DG_OVER_DP, keep) = rec;
         A(b, AGG_TIME, keep) = time;
         if (key != cell_k || fcell != fine_k) regrid_to(b, keep, key, fcell);
-        if (dbits(rmax) > dbits(sc->maxradius)) sc->maxradius = rmax;
+        if (dkey(rmax) > dkey(sc->maxradius) && !is_nan(sc->maxradius)) sc->maxradius = rmax;
         sm.merged = 1;
         st.c_merged_spheres += n;
         st.c_merge_pairs += Pc;

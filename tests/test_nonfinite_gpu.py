@@ -1,0 +1,63 @@
+"""Contact queries on boxes that hold infinite and NaN coordinates.
+
+The swept test compares bit patterns, and a NaN made by the GPU has its sign
+bit set (an infinite coordinate makes one in the periodic distance), so it
+must not order below the contact distance: a sphere without a finite place
+touches nothing, as in the oracle. The FP32 screens drop such spheres for
+short sweeps; a sweep of more than a box length hands every pair to the swept
+test. Single queries and both forms of a batch.
+"""
+import numpy as np
+import pytest
+
+from conftest import load_golden
+from mcac_gb300 import AggregatList, PhysicalModel
+from mcac_gb300.snapshot import A, S, Snapshot
+from mcac_gb300.workloads import random_directions
+from oracle import oracle_py as O
+
+NEGATIVE_NAN = np.array([-0x8000000000000], dtype=np.int64).view(np.float64)[0]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("centres", [False, True])
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, NEGATIVE_NAN], ids=["inf", "-inf", "nan", "-nan"])
+@pytest.mark.parametrize("boxes", [0.1, 1.2])
+@pytest.mark.parametrize("fixture", ["c1_q5000.npz", "ln_late.npz"])
+def test_spheres_without_a_place_touch_nothing(fixture, boxes, value, centres):
+    g = load_golden(fixture)
+    snap = Snapshot.from_npz(g, "s_")
+    ini = str(g["ini"])
+    rng = np.random.Generator(np.random.PCG64(int(10 * boxes) + 31))
+    lost = np.arange(1, snap.na, 3)  # these aggregates' spheres lose a coordinate
+    # (the oracle's wrap loops end for a NaN only, and its cells need finite
+    # centres: it keeps those, and has a NaN for every lost coordinate)
+    ref_snap = snap.copy()
+    for a in lost:
+        snap.spheres[S["x"] + a % 3, snap.members_of(a)] = value
+        ref_snap.spheres[S["x"] + a % 3, snap.members_of(a)] = np.nan
+    ob = O.OracleBox(ini, ref_snap)
+    if centres:
+        snap.aggregates[A["x"] + lost % 3, lost] = value
+    labels = rng.choice(np.setdiff1d(np.arange(snap.na), lost), 12)
+    dirs = random_directions(rng, 12)
+    length = boxes * snap.box_length
+    ref = [ob.distance_to_next_contact(int(l), d, length) for l, d in zip(labels, dirs)]
+    with AggregatList(PhysicalModel(text=ini), snap) as box:
+        one = [box.distance_to_next_contact(int(l), d, length) for l, d in zip(labels, dirs)]
+        few, _ = box.distance_to_next_contacts(labels, dirs, np.full(12, length))
+        many, _ = box.distance_to_next_contacts(np.tile(labels, 60), np.tile(dirs, (60, 1)), np.full(720, length))
+    for k, r in enumerate(ref):
+        got = [one[k]] + [_Row(b[k]) for b in (few, many[:12], many[-12:])]
+        for c in got:
+            assert np.float64(c.distance).view(np.int64) == np.float64(r.distance).view(np.int64)
+            if np.isfinite(r.distance):
+                assert (c.moving_sphere, c.other_sphere, c.other_aggregate) == (
+                    r.moving_sphere, r.other_sphere, r.other_aggregate)
+    assert any(np.isfinite(r.distance) for r in ref) or boxes < 1.0
+
+
+class _Row:
+    def __init__(self, row):
+        for f in ("distance", "moving_sphere", "other_sphere", "other_aggregate"):
+            setattr(self, f, row[f])
