@@ -236,6 +236,7 @@ __device__ __forceinline__ double dkey_inv(unsigned long long k) {
 __device__ __forceinline__ long long dbits(double v) { return __double_as_longlong(v); }
 constexpr unsigned long long kInfBits = 0x7ff0000000000000ULL;
 __device__ __forceinline__ bool is_nan(double v) { return ((unsigned long long)dbits(v) << 1) > (kInfBits << 1); }
+__device__ __forceinline__ bool is_finite(double v) { return ((unsigned long long)dbits(v) << 1) < (kInfBits << 1); }
 // |a| < b for b > 0 (false for a NaN)
 __device__ __forceinline__ bool abs_lt(double a, double b) {
     return (dbits(a) & 0x7fffffffffffffffLL) < dbits(b);

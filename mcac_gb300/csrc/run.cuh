@@ -1581,7 +1581,8 @@ __device__ inline void apply_query(RunState &st, RS &sm, const QueryOut &q) {
         st.status = q.status;
         sm.stop = 1;
     }
-    sm.contact = q.distance <= sm.full;
+    // (a contact has a partner: an infinite length reaches an infinite distance)
+    sm.contact = q.other_slot >= 0 && q.distance <= sm.full;
     sm.move = sm.contact ? q.distance : sm.full;
     sm.ms = q.moving_sphere;
     sm.os = q.other_sphere;

@@ -636,7 +636,7 @@ __device__ __forceinline__ int warp_steps(LS &sm, int phase, unsigned &t_phase) 
                     status = o.status;
                     break;
                 }
-                if (dkey(o.distance) <= dkey(full)) {
+                if (o.oslot >= 0 && dkey(o.distance) <= dkey(full)) {
                     contact = 1;
                     move = o.distance;
                     if (lane == 0) {
@@ -1157,7 +1157,7 @@ __device__ inline void block_rounds(LS &sm, long long max_steps) {
                     if (R.lim.with_collisions && !loop_query(sm, wid, slot, rec, dl, full, o)) heavy = 1;
                     if (R.phys.growth || n > kWarpMove) heavy |= 2;
                 }
-                const int contact = dkey(o.distance) <= dkey(full);
+                const int contact = o.oslot >= 0 && dkey(o.distance) <= dkey(full);
                 const double move = contact ? o.distance : full;
                 const bool sound = slot >= 0 && o.status == ST_OK;
                 if (sound && heavy == 0) mv = loop_prepare(sm, rec, dl, move);

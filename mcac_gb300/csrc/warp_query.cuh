@@ -152,6 +152,8 @@ __device__ __forceinline__ bool warp_query(const DevBox &b, const DevScalars *sc
                                            int src, const WarpRec &rec, double dl, double full, WarpAnswer &o) {
     const int lane = threadIdx.x & 31;
     const unsigned all = 0xffffffffu;
+    // the comparisons with the length below order its bits
+    if (!is_finite(full)) return false;
     // FP32 forms of the direction (lanes 0-2), the length and the largest
     // r_max: one conversion for all of them
     const float cf = float(lane == 3 ? full : (lane == 4 ? sc->maxradius : dl));

@@ -11,7 +11,7 @@ import numpy as np
 import pytest
 
 from conftest import load_golden
-from mcac_gb300 import AggregatList, PhysicalModel
+from mcac_gb300 import AggregatList, Batch, PhysicalModel, StateBuffers
 from mcac_gb300.snapshot import A, S, Snapshot
 from mcac_gb300.workloads import random_directions
 from oracle import oracle_py as O
@@ -61,3 +61,34 @@ class _Row:
     def __init__(self, row):
         for f in ("distance", "moving_sphere", "other_sphere", "other_aggregate"):
             setattr(self, f, row[f])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("collisions", ["true", "false"])
+@pytest.mark.parametrize("value", [np.inf, np.nan, NEGATIVE_NAN], ids=["inf", "nan", "-nan"])
+def test_steps_without_a_finite_length_meet_nothing(value, collisions):
+    models = [PhysicalModel(text=(
+        f"[monomers]\nnumber = {n}\nmean_diameter = 30\ndispersion_diameter = 1.3\ninitialisation_mode = lognormal\n"
+        f"[environment]\nvolume_fraction = 5e-3\ntemperature = 1700\n[limits]\nnumber_of_aggregates = 1\n"
+        f"[numerics]\nrandom_seed = {n}\nwith_domain_duplication = false\nwith_collisions = {collisions}\n"))
+        for n in (60, 90)]
+    with Batch(models) as b:
+        snaps = b.store_all()
+    for s in snaps:
+        s.aggregates[A["lpm"], ::3] = value
+    ends = []
+    for threads in (32, 128, 256, 512):
+        with Batch(models, states=[StateBuffers.from_snapshot(s) for s in snaps]) as b:
+            b.threads = threads
+            b.run(max_steps=100, steps_per_launch=100)
+            st = b.stats()
+            assert np.all(st["status"] == 0) and np.all(st["steps"] == 100)
+            assert np.array_equal(st["events"], [s.na for s in snaps] - st["n_aggregates"])
+            ends.append((st, b.store_all()))
+    for st, out in ends[1:]:
+        for f in ("events", "n_aggregates", "time"):
+            assert np.array_equal(st[f], ends[0][0][f]), f
+        for x, y in zip(out, ends[0][1]):
+            assert np.array_equal(x.spheres, y.spheres, equal_nan=True)
+            assert np.array_equal(x.members, y.members) and np.array_equal(x.sphere_label, y.sphere_label)
+    assert collisions == "true" or not ends[0][0]["events"].any()
