@@ -194,6 +194,11 @@ __device__ __forceinline__ int wrap_cell(int i, int n) {
     return i;
 }
 
+// The start of a cell range, moved by whole boxes to where wrap_cell takes every
+// cell of the range (less than n of them) and every difference of a cell and
+// the start. Only a centre outside the box needs it.
+__device__ __forceinline__ int near_cell(int lo, int n) { return lo >= -n && lo <= n ? lo : periodic_cell(lo, n); }
+
 static __device__ __noinline__ void neighborhood_axis_call(double s, double v, double distance, int n_div, double width,
                                                     double inv_width, int *lo, int *hi) {
     neighborhood_axis(s, v, distance, n_div, width, inv_width, lo, hi);
@@ -550,13 +555,16 @@ __device__ inline void block_query(const DevBox &b, int src, Vec3 dir, double di
                 const double sl = tid == 0 ? sp.x : (tid == 1 ? sp.y : sp.z);
                 neighborhood_axis_call(sl, dist * dl, rmax_src + sc->maxradius, b.n_div, b.L, b.inv_L, &lo, &hi);
             }
+            const int near = near_cell(lo, b.n_div);
+            hi += near - lo;
+            lo = near;
             sm.range.lo[tid] = lo;
             sm.range.hi[tid] = hi;
             if (b.fine_div > 0) {
                 const float flof = floorf((pf - mf + fminf(vf, 0.f)) * b.fine_step_f - 2e-3f);
                 const float fhif = floorf((pf + mf + fmaxf(vf, 0.f)) * b.fine_step_f + 2e-3f);
                 const bool part = (fhif - flof + 1.f < float(b.fine_div)) && flof > -1e6f && fhif < 1e6f;
-                flo = part ? int(flof) : 0;
+                flo = part ? near_cell(int(flof), b.fine_div) : 0;
                 fn = part ? int(fhif - flof + 1.f) : b.fine_div;
                 sm.fine_lo[tid] = flo;
                 sm.fine_n[tid] = fn;

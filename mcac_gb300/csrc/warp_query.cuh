@@ -186,11 +186,12 @@ __device__ __forceinline__ bool warp_query(const DevBox &b, const DevScalars *sc
         if (!neighborhood_axis_f32(pf, vf, reach_f, b.n_div, b.step_f, &lo, &hi))
             neighborhood_axis_call(x_ax, full * dl, rmax + sc->maxradius, b.n_div, b.L, b.inv_L, &lo, &hi);
         n_c = hi - lo + 1;
+        lo = near_cell(lo, b.n_div);
         if (b.fine_div > 0) {  // widened as in block_query
             const float flof = floorf((pf - reach_f + fminf(vf, 0.f)) * b.fine_step_f - 2e-3f);
             const float fhif = floorf((pf + reach_f + fmaxf(vf, 0.f)) * b.fine_step_f + 2e-3f);
             const bool part = (fhif - flof + 1.f < float(b.fine_div)) && flof > -1e6f && fhif < 1e6f;
-            flo = part ? int(flof) : 0;
+            flo = part ? near_cell(int(flof), b.fine_div) : 0;
             fn = part ? int(fhif - flof + 1.f) : b.fine_div;
         }
     }

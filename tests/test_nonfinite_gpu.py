@@ -12,6 +12,7 @@ import pytest
 
 from conftest import load_golden
 from mcac_gb300 import AggregatList, Batch, PhysicalModel, StateBuffers
+from mcac_gb300._lib import MCACError
 from mcac_gb300.snapshot import A, S, Snapshot
 from mcac_gb300.workloads import random_directions
 from oracle import oracle_py as O
@@ -61,6 +62,38 @@ class _Row:
     def __init__(self, row):
         for f in ("distance", "moving_sphere", "other_sphere", "other_aggregate"):
             setattr(self, f, row[f])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("boxes", [0, 1, -1, 7, -40, 100000])
+@pytest.mark.parametrize("fixture", ["c1_q5000.npz", "ln_late.npz"])
+def test_one_query_and_a_batch_agree_on_centres_outside_the_box(fixture, boxes):
+    """A state's centres are not checked when it is loaded. The source of the
+    query and its spheres lie whole boxes away: its cells are taken modulo the
+    grid, and both forms of the query find the same (the Verlet grid files the
+    centre under its nearest cell, so most often: that it is not listed)."""
+    g = load_golden(fixture)
+    snap = Snapshot.from_npz(g, "s_")
+    rng = np.random.Generator(np.random.PCG64(77))
+    labels = rng.choice(snap.na, 10, replace=False)
+    for l in labels:
+        snap.aggregates[A["x"]:A["z"] + 1, l] += boxes * snap.box_length
+        snap.spheres[:3, snap.members_of(l)] += boxes * snap.box_length
+    found = 0
+    with AggregatList(PhysicalModel(text=str(g["ini"])), snap) as box:
+        for l, d in zip(labels, random_directions(rng, 10)):
+            for length in (1e-3 * snap.box_length, 0.3 * snap.box_length, snap.box_length):
+                got = []
+                for ask in (lambda: box.distance_to_next_contact(int(l), d, length),
+                            lambda: _Row(box.distance_to_next_contacts([l], [d], [length])[0][0])):
+                    try:
+                        c = ask()
+                        got.append((c.distance, c.moving_sphere, c.other_sphere, c.other_aggregate))
+                    except MCACError as e:
+                        got.append(e.code)
+                assert got[0] == got[1]
+                found += not isinstance(got[0], int)
+    assert boxes != 0 or found == 30
 
 
 @pytest.mark.gpu
