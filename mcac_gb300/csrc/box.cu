@@ -135,9 +135,11 @@ __global__ void __launch_bounds__(32 * kQueryWarps, 4) k_query_warps(DevBox b, B
     }
 }
 
-// Large queries, a block each (s.left lists them; all n queries when it is
-// null). 256 threads: what is left here are long pair searches, and the
-// batch ends with the longest.
+// Queries by blocks, a block each: those that the warps left (s.left lists
+// them), or all n (s.left null). 256 threads shorten the longest pair
+// searches, with which most batches end; 128 keep twice as many queries in
+// flight, which pays for more queries than such blocks are resident
+// (query_batch).
 template <int NT>
 __global__ void __launch_bounds__(NT, 512 / NT) k_query_batch(DevBox b, BatchScratch s, int n, const QueryIn *in,
                                                               QueryOut *out) {
@@ -1383,8 +1385,35 @@ int DeviceBox::query(int src_slot, const double dir[3], double dist, QueryResult
     return q.status;
 }
 
-int DeviceBox::query_batch(int n, const int *slots, const double *dirs, const double *dists, QueryResult *out,
-                           double *kernel_ms, std::string *err) {
+// Which kernels answer a batch of n queries, from the spheres per live
+// aggregate (what a query's pairs grow with) and n. Kernel time in us, by
+// warps first with the rest by blocks / by blocks of 256 / of 128 threads
+// (geometric means of three synthetic states; before: 'warps from 609 queries
+// on, else 256'):
+//   spheres   n = 64       n = 600      n = 1500       n = 3000       n = 10 000
+//      1     20/ 30/ 27   24/ 37/ 31   24/ 53/ 40     28/ 83/ 55     39/210/119
+//      3     21/ 30/ 28   26/ 42/ 33   28/ 64/ 44     32/103/ 66     46/280/156
+//     10     60/ 41/ 46   74/ 48/ 49   73/ 73/ 75     94/127/ 99    135/330/200
+//     25     84/ 41/ 45  128/ 74/ 72  135/ 91/ 86    159/156/121    214/350/234
+//     50     82/ 44/ 49  132/ 88/ 95  203/154/161    229/209/182    322/411/312
+//    100    139/ 92/ 95  184/135/167  189/146/175    216/198/194    399/442/390
+//    400    102/ 95/127  165/157/173  193/186/203    247/238/238
+//   1000     32/ 25/ 27   44/ 35/ 33   70/ 61/ 48    111/ 98/ 72
+//   1333     73/ 60/ 80   91/ 81/ 97  128/117/121    210/194/175
+// A warp leaves most queries of larger aggregates to the blocks, so its pass
+// is lost there; for enough of them it still saves the blocks the rest.
+struct BatchPlan {
+    bool warps;
+    int threads;  // of the blocks
+};
+BatchPlan batch_plan(int n, double mean_members, int n_sm) {
+    const bool warps = mean_members <= 5.0 || double(n) >= 128.0 * mean_members;
+    // more than two queries for each resident block of 128 threads (four an SM)
+    return BatchPlan{warps, !warps && n > 2 * 4 * n_sm ? 128 : 256};
+}
+
+int DeviceBox::query_batch(int n, const int *slots, const double *dirs, const double *dists, double mean_members,
+                           QueryResult *out, double *kernel_ms, std::string *err) {
     if (kernel_ms) *kernel_ms = 0.0;
     if (n <= 0) return ST_OK;
     for (int k = 0; k < n; ++k)
@@ -1406,13 +1435,15 @@ int DeviceBox::query_batch(int n, const int *slots, const double *dirs, const do
                    cuda_ok(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100), err,
                            "cudaFuncSetAttribute");
         };
-        if (!set((const void *)k_query_batch<256>)) return ST_CUDA;
+        if (!set((const void *)k_query_batch<128>) || !set((const void *)k_query_batch<256>)) return ST_CUDA;
         attrs = true;
     }
-    constexpr int kThreads = 256;
+    const BatchPlan plan = batch_plan(n, mean_members, n_sm);
     int per_sm = 0;
-    if (!cuda_ok(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_query_batch<kThreads>, kThreads,
-                                                               sizeof(QuerySmem)),
+    if (!cuda_ok(plan.threads == 128 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_query_batch<128>, 128,
+                                                                                     sizeof(QuerySmem))
+                                     : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_query_batch<256>, 256,
+                                                                                     sizeof(QuerySmem)),
                  err, "occupancy"))
         return ST_CUDA;
     const int blocks = std::max(1, std::min(n, std::max(1, per_sm) * std::max(1, n_sm)));
@@ -1475,19 +1506,19 @@ int DeviceBox::query_batch(int n, const int *slots, const double *dirs, const do
                       "query upload") &&
               cuda_ok(cudaMemsetAsync(sc.next, 0, 3 * sizeof(int), s), err, "query counter");
     if (ok) {
-        // the small queries by warps, then the rest of them by blocks; calls
-        // of at most two queries for each block the GPU runs at once go to the
-        // blocks directly (500 queries of large aggregates: 199 -> 208 us with
-        // the warps first, 167 -> 159 us without; 10 000 queries on a million
-        // spheres 836 -> 710 us with them)
+        // the small queries by warps, then the rest of them by blocks; or all
+        // by blocks (batch_plan)
         cudaEventRecord(e0, s);
-        if (n > 2 * blocks) {
+        if (plan.warps) {
             const int grid = std::min((n + kQueryWarps - 1) / kQueryWarps, 4 * std::max(1, n_sm));
             k_query_warps<<<grid, 32 * kQueryWarps, 0, s>>>(b, sc, n, sc.next + 2, d_in, d_out);
         } else {
             sc.left = nullptr;
         }
-        k_query_batch<kThreads><<<blocks, kThreads, sizeof(QuerySmem), s>>>(b, sc, n, d_in, d_out);
+        if (plan.threads == 128)
+            k_query_batch<128><<<blocks, 128, sizeof(QuerySmem), s>>>(b, sc, n, d_in, d_out);
+        else
+            k_query_batch<256><<<blocks, 256, sizeof(QuerySmem), s>>>(b, sc, n, d_in, d_out);
         cudaEventRecord(e1, s);
         ok = cuda_ok(cudaGetLastError(), err, "k_query_batch") &&
              cuda_ok(cudaMemcpyAsync(hout.data(), d_out, sizeof(QueryOut) * size_t(n), cudaMemcpyDeviceToHost, s), err,

@@ -148,11 +148,12 @@ class DeviceBox {
     bool owns_stream() const { return own_stream_; }
     int query(int src_slot, const double dir[3], double dist, QueryResult *out, std::string *err);
     // n independent queries on the current state (nothing is moved): slots[k],
-    // dirs[3k..3k+2], dists[k] -> out[k]. The queries run concurrently, one
-    // per thread block. Returns the first failing status, or ST_OK;
-    // *kernel_ms (may be null) gets the kernel's CUDA-event time.
-    int query_batch(int n, const int *slots, const double *dirs, const double *dists, QueryResult *out,
-                    double *kernel_ms, std::string *err);
+    // dirs[3k..3k+2], dists[k] -> out[k]. The queries run concurrently, a warp
+    // or a thread block each; 'mean_members', the spheres per live aggregate,
+    // only chooses between these. Returns the first failing status, or ST_OK;
+    // *kernel_ms (may be null) gets the kernels' CUDA-event time.
+    int query_batch(int n, const int *slots, const double *dirs, const double *dists, double mean_members,
+                    QueryResult *out, double *kernel_ms, std::string *err);
     int translate(int slot, const double v[3], std::string *err);
     int merge(int ms, int os, int mslot, int oslot, MergeResult *out, std::string *err);
     // Writes aggregate fields of one slot: fields[f] for every f with bit f of mask set.

@@ -585,7 +585,8 @@ int HostBox::distance_to_next_contacts(int n, const int64_t *labels, const doubl
         slots[size_t(k)] = alive_[size_t(labels[k])];
     }
     std::vector<QueryResult> q(static_cast<size_t>(n));
-    int rc = dev_->query_batch(n, slots.data(), dirs, distances, q.data(), kernel_ms, err);
+    const double mean_members = double(ns_) / double(std::max<size_t>(1, alive_.size()));
+    int rc = dev_->query_batch(n, slots.data(), dirs, distances, mean_members, q.data(), kernel_ms, err);
     for (int k = 0; k < n; ++k) {
         const QueryResult &r = q[size_t(k)];
         mcacg_contact &c = out[k];
