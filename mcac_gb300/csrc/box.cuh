@@ -315,15 +315,19 @@ static __device__ __noinline__ double sweep_contact_general(Vec3 p1, double r1, 
 // 60 FP64 instructions instead of about 160 (three divisions, three fmod
 // and some twenty comparisons less). Together with the FP32 cell range:
 // 10 000 queries on a million spheres 782 -> 728 us, single queries 20.3 ->
-// 18.8 us, the 512-box ensemble's step 39.5 -> 35.8 us.
-static __device__ __noinline__ double sweep_contact_fast(Vec3 p1, double r1, Vec3 p2, double r2, Vec3 dir, double dist,
-                                                         double L) {
+// 18.8 us, the 512-box ensemble's step 39.5 -> 35.8 us. 'InLine': the wrap
+// loops, the general routine and the square root in line too, so that there is
+// no call.
+template <bool InLine>
+__device__ __forceinline__ double sweep_contact_short(Vec3 p1, double r1, Vec3 p2, double r2, Vec3 dir, double dist,
+                                                      double L) {
+    auto distance = [L](double d) { return InLine ? periodic_distance(d, L) : wrap_distance(d, L); };
     const double dc = r1 + r2;
     const double dc2 = dc * dc;
     {
-        const double dx = wrap_distance(p1.x - p2.x, L);
-        const double dy = wrap_distance(p1.y - p2.y, L);
-        const double dz = wrap_distance(p1.z - p2.z, L);
+        const double dx = distance(p1.x - p2.x);
+        const double dy = distance(p1.y - p2.y);
+        const double dz = distance(p1.z - p2.z);
         if (nonneg_le(dx * dx + dy * dy + dz * dz, dc2)) return 0.0;
     }
     const double pa[3] = {p1.x, p1.y, p1.z}, pb[3] = {p2.x, p2.y, p2.z}, u[3] = {dir.x, dir.y, dir.z};
@@ -349,7 +353,9 @@ static __device__ __noinline__ double sweep_contact_fast(Vec3 p1, double r1, Vec
         d[l] = q[l] - pa[l];
         outside = outside || (dbits(d[l]) & 0x7fffffffffffffffLL) > dbits(zone);
     }
-    if (!usual) return sweep_contact_general(p1, r1, p2, r2, dir, dist, L);
+    if (!usual)
+        return InLine ? sweep_contact_distance(p1, r1, p2, r2, dir, dist, L)
+                      : sweep_contact_general(p1, r1, p2, r2, dir, dist, L);
     const double inf = CUDART_INF;
     if (outside) return inf;
     const double proj = d[0] * u[0] + d[1] * u[1] + d[2] * u[2];
@@ -362,7 +368,11 @@ static __device__ __noinline__ double sweep_contact_fast(Vec3 p1, double r1, Vec
     const double cz = d[0] * u[1] - d[1] * u[0];
     const double axis = cx * cx + cy * cy + cz * cz;
     if (!nonneg_le(axis, dc2)) return inf;
-    return proj - fp64_sqrt(dc2 - axis);
+    return proj - (InLine ? sqrt(dc2 - axis) : fp64_sqrt(dc2 - axis));
+}
+static __device__ __noinline__ double sweep_contact_fast(Vec3 p1, double r1, Vec3 p2, double r2, Vec3 dir, double dist,
+                                                         double L) {
+    return sweep_contact_short<false>(p1, r1, p2, r2, dir, dist, L);
 }
 
 // Conservative FP32 capsule test: can a sphere at p2 (radius folded into
@@ -924,13 +934,15 @@ __device__ inline void block_query(const DevBox &b, int src, Vec3 dir, double di
         if (!capsule_hit(wi, q.x, q.y, q.z, p.w + q.w + margin)) return;
         const int si = pool_id[off_m + t0 + i];
         const int sj = pool_id[pj];
-        // The general form, in line: with sweep_contact_fast, a call, or with
-        // its body in line the FP32 screens around it spill more, and late
-        // searches took longer than before it (500 queries on aggregates of
-        // 1333 spheres, kernel: 308 us before, 332 with the call, 300 with its
-        // body in line, 264 so; of 100 spheres 144, 98, 98 and 84).
-        const double res = sweep_contact_distance(sph_pos(b, si), S(b, SPH_R, si), sph_pos(b, sj), S(b, SPH_R, sj), dir,
-                                                  dist, b.L);
+        // In line with all that it may call: around a call the FP32 screens
+        // spill more, and late searches took longer than with the general
+        // form in line, before the short one was there (500 queries on
+        // aggregates of 1333 spheres, kernel: 308 us then, 332 with a call,
+        // 300 with the short form in line and calls in it; 100 of ten
+        // spheres 33 us with a call, 35 with the general form in line, 30 so;
+        // 450 of 250 spheres 271, 232 and 234).
+        const double res = sweep_contact_short<true>(sph_pos(b, si), S(b, SPH_R, si), sph_pos(b, sj), S(b, SPH_R, sj),
+                                                     dir, dist, b.L);
         atomicAdd(&sm.n_refined, 1);
         if (!(res < CUDART_INF)) return;
         unsigned long long key = dkey(res);
