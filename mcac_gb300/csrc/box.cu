@@ -1385,29 +1385,32 @@ int DeviceBox::query(int src_slot, const double dir[3], double dist, QueryResult
     return q.status;
 }
 
-// Which kernels answer a batch of n queries, from the spheres per live
-// aggregate (what a query's pairs grow with) and n. Kernel time in us, by
-// warps first with the rest by blocks / by blocks of 256 / of 128 threads
-// (geometric means of three synthetic states; before: 'warps from 609 queries
-// on, else 256'):
-//   spheres   n = 64       n = 600      n = 1500       n = 3000       n = 10 000
-//      1     20/ 30/ 27   24/ 37/ 31   24/ 53/ 40     28/ 83/ 55     39/210/119
-//      3     21/ 30/ 28   26/ 42/ 33   28/ 64/ 44     32/103/ 66     46/280/156
-//     10     60/ 41/ 46   74/ 48/ 49   73/ 73/ 75     94/127/ 99    135/330/200
-//     25     84/ 41/ 45  128/ 74/ 72  135/ 91/ 86    159/156/121    214/350/234
-//     50     82/ 44/ 49  132/ 88/ 95  203/154/161    229/209/182    322/411/312
-//    100    139/ 92/ 95  184/135/167  189/146/175    216/198/194    399/442/390
-//    400    102/ 95/127  165/157/173  193/186/203    247/238/238
-//   1000     32/ 25/ 27   44/ 35/ 33   70/ 61/ 48    111/ 98/ 72
-//   1333     73/ 60/ 80   91/ 81/ 97  128/117/121    210/194/175
+// Which kernels answer a batch of n queries, from n and the spheres per live
+// aggregate (what a query's pairs grow with). Kernel time in us, by warps
+// first with the rest by blocks of 256 threads / by blocks of 256 / of 128
+// (geometric means over three synthetic states):
+//   spheres   n = 64       n = 600      n = 1500     n = 3000     n = 5000     n = 10 000
+//      1     20/ 27/ 25   24/ 35/ 30   24/ 51/ 37   28/ 80/ 53   31/116/ 71   39/204/115
+//      3     21/ 28/ 26   27/ 38/ 30   28/ 61/ 42   32/ 98/ 63   42/149/ 88   46/273/150
+//     10     58/ 35/ 38   73/ 43/ 41   73/ 67/ 60   93/119/ 85  107/172/103  122/320/186
+//     25     82/ 35/ 37  122/ 68/ 66  127/ 80/ 76  154/151/117  169/185/136  203/332/212
+//     50     82/ 38/ 44  131/ 80/ 94  204/154/162  229/205/180  249/272/230  320/406/303
+//    100    141/ 93/ 96  184/135/167  190/147/178  217/199/190  264/259/227  399/442/390
+//    400    105/ 98/127  164/157/177  196/189/205  251/241/242
+//   1000     33/ 24/ 27   45/ 35/ 34   71/ 61/ 49  112/ 99/ 73
+//   1333     74/ 62/ 78   92/ 81/ 98  129/119/121  212/195/176
 // A warp leaves most queries of larger aggregates to the blocks, so its pass
-// is lost there; for enough of them it still saves the blocks the rest.
+// is lost on them, unless the batch is so large that it keeps enough from the
+// blocks. Many queries fill the SMs with blocks of 128 threads; of few, the
+// longest pair search decides, which 256 threads shorten. (One line at 608
+// queries, warps above and blocks of 256 below, took 208 us for 700 queries
+// on aggregates of 100 spheres, now 140.)
 struct BatchPlan {
     bool warps;
     int threads;  // of the blocks
 };
 BatchPlan batch_plan(int n, double mean_members, int n_sm) {
-    const bool warps = mean_members <= 5.0 || double(n) >= 128.0 * mean_members;
+    const bool warps = mean_members <= 5.0 || double(n) >= 400.0 * mean_members;
     // more than two queries for each resident block of 128 threads (four an SM)
     return BatchPlan{warps, !warps && n > 2 * 4 * n_sm ? 128 : 256};
 }
