@@ -139,7 +139,7 @@ struct RunSmemT {
         QS q;
         MS m;
         WarpQueryScratch<256, 1024> w;
-        WarpQueryScratch<192, 1024> r[Rounds];  // one for each step of a round
+        WarpQueryScratch<192, 1024, QueryLists> r[Rounds];  // one for each step of a round
         WarpMergeScratch wm;
     } u;
     MergeOut mout;

@@ -1044,6 +1044,40 @@ __device__ inline void rounds_decide(LS &sm, unsigned t_start) {
     __syncwarp();
 }
 
+// A warp without a step, while the others carry out theirs: a query read its
+// lists as they were at the round's start, so what the earlier steps of the
+// round moved into or out of them is added to the count of scanned aggregates,
+// which is then that of the steps one after another.
+template <class LS>
+__device__ inline void rounds_count(LS &sm) {
+    const int lane = threadIdx.x & 31, c = sm.n_commit;
+    const DevBox &b = sm.R.box;
+    int pj = 1;  // pairs as in rounds_decide
+    while (lane >= (pj * (pj + 1)) / 2) ++pj;
+    int listed = 0;
+    if (pj < c && !sm.live.on) {
+        const RoundJob &x = sm.job[lane - (pj * (pj - 1)) / 2];
+        const QueryLists &y = sm.u.r[pj].lists;
+        auto in = [&](int i, int j, int k, int n) {
+            return int(wrap_cell(i - y.axis[0].x, n) < (y.axis[0].y & (kFineLists - 1)) &&
+                       wrap_cell(j - y.axis[1].x, n) < (y.axis[1].y & (kFineLists - 1)) &&
+                       wrap_cell(k - y.axis[2].x, n) < (y.axis[2].y & (kFineLists - 1)));
+        };
+        auto verlet = [&](int key) { return in(key & 1023, (key >> 10) & 1023, key >> 20, b.n_div); };
+        auto fine = [&](int cell) {
+            const int n = b.fine_div, row = cell / n;
+            return in(row / n, row % n, cell % n, n);
+        };
+        if (y.axis[0].y & kFineLists) {
+            if (x.fine != x.old_fine) listed = fine(x.fine) - fine(x.old_fine);
+        } else if (x.key != x.old_key) {
+            listed = verlet(x.key) - verlet(x.old_key);
+        }
+    }
+    listed = __reduce_add_sync(0xffffffffu, listed);
+    if (lane == 0 && sm.R.lim.with_collisions) sm.st.c_scanned += listed;
+}
+
 template <class LS>
 __device__ __noinline__ int warp_steps_call(int phase, unsigned t_phase) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1322,6 +1356,7 @@ __device__ inline void block_rounds(LS &sm, long long max_steps) {
                 t_phase = clock_lo();
                 __syncthreads();
                 const int c = sm.n_commit;
+                if (wid == kMax) rounds_count(sm);  // (256 threads and more: a warp beyond the round's)
                 if (wid < c) {
                     loop_move_call<LS>(slot, rec, mv, !((sm.serial >> wid) & 1));
                     const double dt = wid == c - 1 ? sm.commit_dt : st.inv_weight;

@@ -8,6 +8,8 @@
 // per swept test, one axis each. Queries beyond the scratch (long neighbour
 // lists, many sphere pairs) are left to block_query; both give the same bits.
 #pragma once
+#include <type_traits>
+
 #include "box.cuh"
 
 namespace mcacg {
@@ -15,12 +17,23 @@ namespace mcacg {
 constexpr int kWarpCells = 128;  // cells a query visits (four per lane)
 constexpr int kWarpCands = 32;   // neighbours past the FP32 screen; sphere pairs to refine
 
+// The cells that a query read, an axis each: x the first (periodic), y how many
+// of them, plus kFineLists when they are fine cells, not Verlet cells. (One
+// store for three lanes: what a round notes costs every query of it.)
+constexpr int kFineLists = 1 << 16;
+struct QueryLists {
+    int2 axis[3];
+};
+struct NoQueryLists {};
+
 // Scratch of a one-warp query: up to Queue aggregates listed and Pairs sphere
-// pairs screened.
-template <int Queue, int Pairs>
+// pairs screened. 'Lists' (QueryLists): the query notes the lists it read.
+template <int Queue, int Pairs, class Lists = NoQueryLists>
 struct WarpQueryScratch {
     static constexpr int kQueue = Queue;
     static constexpr int kPairs = Pairs;
+    static constexpr bool kNotesLists = !std::is_same<Lists, NoQueryLists>::value;
+    Lists lists;
     int queue[Queue];
     // neighbours past the FP32 screen, with their scan keys
     int scr_slot[kWarpCands];
@@ -220,6 +233,9 @@ __device__ __forceinline__ bool warp_query(const DevBox &b, const DevScalars *sc
         }
         const int n_cells = fine ? n_fine : n_scan;
         if (n_cells > kWarpCells) return false;
+        if constexpr (WS::kNotesLists) {
+            if (lane < 3) W.lists.axis[lane] = fine ? make_int2(flo, fn | kFineLists) : make_int2(lo, n_c);
+        }
         o.cells = n_cells;
         const int dy = fine ? fn1 : ny, dz = fine ? fn2 : nz, nf = fine ? b.fine_div : nd;
         const int l0 = fine ? shfl_i(flo, 0) : rlo0, l1 = fine ? shfl_i(flo, 1) : rlo1, l2 = fine ? shfl_i(flo, 2) : rlo2;
