@@ -434,6 +434,11 @@ int mcacg_batch_store_states(mcacg_batch *batch, mcacg_state *states, int32_t n_
 int mcacg_batch_work(mcacg_batch *batch, mcacg_profile *out);
 /* The same counters for one box of the batch. */
 int mcacg_batch_box_work(mcacg_batch *batch, int32_t box, mcacg_profile *out);
+/* Diagnostic: the rounds that the device loop took since creation (with 256
+ * threads and more a box's next steps may be answered at once and committed
+ * in order), and the steps committed in them, summed over boxes. How many
+ * there are depends on the clock; the runs do not. */
+int mcacg_batch_rounds(mcacg_batch *batch, int64_t *rounds, int64_t *steps);
 /* GPU time (CUDA events) and kernel launches of the last mcacg_batch_run. */
 int mcacg_batch_last_run(const mcacg_batch *batch, double *kernel_ms, int32_t *launches);
 

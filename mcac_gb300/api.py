@@ -451,6 +451,12 @@ class Batch:
         check(lib().mcacg_batch_work(self._b, C.byref(p)))
         return {name: getattr(p, name) for name, _ in _lib.Profile._fields_}
 
+    def rounds(self) -> tuple[int, int]:
+        """(rounds, steps committed in them) of the device loop since creation."""
+        n, steps = C.c_int64(), C.c_int64()
+        check(lib().mcacg_batch_rounds(self._b, C.byref(n), C.byref(steps)))
+        return n.value, steps.value
+
     def last_run(self) -> tuple[float, int]:
         ms, n = C.c_double(), C.c_int32()
         check(lib().mcacg_batch_last_run(self._b, C.byref(ms), C.byref(n)))

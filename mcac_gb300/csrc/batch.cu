@@ -954,6 +954,8 @@ int BatchRunner::stats(std::vector<BoxRunStats> *out, std::string *err) {
         o.refined = r.c_refined;
         o.merged_spheres = r.c_merged_spheres;
         o.merge_pairs = r.c_merge_pairs;
+        o.rounds = r.c_rounds;
+        o.round_steps = r.c_round_steps;
         o.cyc_pick = r.cyc_pick;
         o.cyc_query = r.cyc_query;
         o.cyc_move = r.cyc_move;

@@ -922,6 +922,22 @@ int mcacg_batch_box_work(mcacg_batch *batch, int32_t box, mcacg_profile *out) {
     });
 }
 
+int mcacg_batch_rounds(mcacg_batch *batch, int64_t *rounds, int64_t *steps) {
+    return guarded([&] {
+        if (!batch || !rounds || !steps) return fail(MCACG_ERR_BAD_ARGUMENT, "null argument");
+        std::vector<mcacg::BoxRunStats> s;
+        std::string err;
+        int rc = batch->impl->stats(&s, &err);
+        if (rc != 0) return finish(rc, err);
+        *rounds = *steps = 0;
+        for (const auto &x : s) {
+            *rounds += x.rounds;
+            *steps += x.round_steps;
+        }
+        return 0;
+    });
+}
+
 int mcacg_server_create(int32_t capacity, int64_t memory_budget_bytes, void *cuda_stream, int32_t keep_final_states,
                         mcacg_server **server) {
     return guarded([&] {

@@ -65,6 +65,7 @@ struct RunState {
     // work counters of the contact queries and merges (algorithmic bytes)
     long long c_queries, c_mov, c_scanned, c_cells, c_candidates, c_cand_spheres, c_refined;
     long long c_merged_spheres, c_merge_pairs;
+    long long c_rounds, c_round_steps;  // rounds taken (step.cuh), and the steps committed in them
     // SM clock cycles spent by the block in each phase of the step
     long long cyc_pick, cyc_query, cyc_move, cyc_merge;
     long long cyc_qscan, cyc_qpairs;  // parts of cyc_query

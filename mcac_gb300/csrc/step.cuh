@@ -991,6 +991,8 @@ __device__ inline void rounds_decide(LS &sm, unsigned t_start) {
     if (lane == 0) {
         sm.n_commit = c;
         sm.round_n += 1;
+        st.c_rounds += 1;
+        st.c_round_steps += c;
         sm.round_sum += first ? 1 : c;
         sm.serial = int(serial);
         sm.commit_dt = last_dt;
