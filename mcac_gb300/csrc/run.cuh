@@ -146,7 +146,6 @@ struct RunSmemT {
     MergeOut mout;
     double refpos[3];
     double dir[3];
-    unsigned long long t_pick;  // pick target in the tree's fixed point
     unsigned long long deadline;  // %globaltimer time after which no step starts (0: none)
     double dt, full, move;
     int slot, contact, stop, merged, rescale;
