@@ -324,16 +324,19 @@ static __device__ __noinline__ void thread_merge_caps(const DevBox &b, const int
 // "alphas" (aggregat.cpp:391-426), one thread: the sums over every contact
 // seen from both spheres (here each pair twice in a row, in (i, j) order),
 // then the corrections.
-static __device__ __noinline__ void alpha_add_call(AlphaSums &a, double r1, double r2, double d) {
+// A pair from both sides: in line, so that the two share their powers (as two
+// calls, merges and updates with this method took up to 1.43 times as long:
+// 300 host-driven steps on 150 aggregates of 20 spheres 38.2 ms, so 26.7).
+__device__ __forceinline__ void alpha_add_both(AlphaSums &a, double r1, double r2, double d) {
     alpha_add(a, r1, r2, d);
+    alpha_add(a, r2, r1, d);
 }
 static __device__ __noinline__ void thread_merge_alphas(const DevBox &b, const int *mem, int n, int P, double *volume,
                                                         double *surface, double *overlap, double *coord) {
     AlphaSums a{0., 0., 0., 0., 0., 0.};
     for (int p = 0; p < P; ++p) {
         const double ri = S(b, SPH_R, mem[b.pair_i[p]]), rj = S(b, SPH_R, mem[b.pair_j[p]]);
-        alpha_add_call(a, ri, rj, b.pair_d[p]);
-        alpha_add_call(a, rj, ri, b.pair_d[p]);
+        alpha_add_both(a, ri, rj, b.pair_d[p]);
     }
     alpha_finish(a, n, 2 * P, volume, surface, overlap, coord);
 }
@@ -732,8 +735,7 @@ static __device__ __noinline__ double thread_update_geometry(const DevBox &b, in
                     b.sph_volw[sj] = b.sph_volw[sj] - k.v2;
                     surf_w[sj] = surf_w[sj] - k.s2;
                 } else if (b.volsurf == VS_ALPHAS) {
-                    alpha_add_call(al, ri, rj, dist);
-                    alpha_add_call(al, rj, ri, dist);
+                    alpha_add_both(al, ri, rj, dist);
                 }
             }
             if (b.volsurf == VS_CAPS) {

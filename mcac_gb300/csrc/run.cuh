@@ -743,8 +743,7 @@ static __device__ __noinline__ double warp_update_geometry(const DevBox &b, int 
                     } else {
                         const double r1 = __shfl_sync(all, ri, src), r2 = __shfl_sync(all, rj, src);
                         const double d2 = __shfl_sync(all, dist, src);
-                        alpha_add_call(al, r1, r2, d2);
-                        alpha_add_call(al, r2, r1, d2);
+                        alpha_add_both(al, r1, r2, d2);
                     }
                 }
             });
