@@ -475,15 +475,27 @@ __device__ __forceinline__ WarpPicked warp_pick(LS &sm, int rnd) {
     return p;
 }
 
-// warp_query on the scratch of the round's step k.
+// warp_query on the scratch of the round's step k. Where the last kMissRun
+// queries of larger aggregates were the block's (dense boxes of few aggregates),
+// the next ones go there without a try, all but every sixteenth.
 template <class LS>
 __device__ __forceinline__ bool loop_query(LS &sm, int k, int src, const WarpRec &rec, double dl, double full,
                                            WarpAnswer &o) {
     const int *live = sm.live.on ? sm.live.slot : nullptr;
-    if constexpr (LS::kRounds > 1)
-        return warp_query(sm.R.box, &sm.sc, sm.u.r[k], live, sm.live.n, src, rec, dl, full, o);
-    else
-        return warp_query(sm.R.box, &sm.sc, sm.u.w, live, sm.live.n, src, rec, dl, full, o);
+    const bool large = shfl_i(rec.i, REC_N) >= kWarpEarly;
+    bool ok = false;
+    if (!large || sm.misses < kMissRun || (sm.misses & 15) == 0) {
+        if constexpr (LS::kRounds > 1)
+            ok = warp_query(sm.R.box, &sm.sc, sm.u.r[k], live, sm.live.n, src, rec, dl, full, o);
+        else
+            ok = warp_query(sm.R.box, &sm.sc, sm.u.w, live, sm.live.n, src, rec, dl, full, o);
+    }
+    if (large && k == 0) {
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) sm.misses = ok ? 0 : sm.misses + 1;
+        __syncwarp();
+    }
+    return ok;
 }
 
 // A picked slot's move, prepared: its place, the members' first ten and what
@@ -844,6 +856,7 @@ struct LoopSmemT : RS {
     RunState st;
     DevScalars sc;
     long long left;  // steps still allowed in this launch
+    int misses;      // queries of larger aggregates in a row that were the block's (loop_query)
     int far;         // block_op: the query's aggregate is the block's to move
     const int *rec_ptr[REC_INTS];  // the integer tables of a slot's record
 };
@@ -1099,6 +1112,7 @@ __device__ inline void block_rounds(LS &sm, long long max_steps) {
     if (threadIdx.x == 0) {
         record_rows_init(b, sm.rec_ptr);
         sm.stop = 0;
+        sm.misses = 0;
         sm.left = max_steps;
         // the criteria may have changed since the last launch; afterwards
         // they are checked at the end of every step
@@ -1401,6 +1415,7 @@ __device__ inline void block_steps(LS &sm, long long max_steps) {
     if (threadIdx.x == 0) {
         record_rows_init(sm.R.box, sm.rec_ptr);
         sm.stop = 0;
+        sm.misses = 0;
         sm.left = max_steps;
         // the criteria may have changed since the last launch; afterwards
         // they are checked at the end of every step

@@ -15,6 +15,7 @@
 namespace mcacg {
 
 constexpr int kWarpCells = 128;  // cells a query visits (four per lane)
+constexpr int kWarpEarly = 8;    // spheres of an aggregate whose pairs are counted before the filter too
 constexpr int kWarpCands = 32;   // neighbours past the FP32 screen; sphere pairs to refine
 
 // The cells that a query read, an axis each: x the first (periodic), y how many
@@ -333,6 +334,15 @@ __device__ __forceinline__ bool warp_query(const DevBox &b, const DevScalars *sc
             total += __popc(mn);
         }
         __syncwarp();
+    }
+    // The screen's spheres bound the filter's: more pairs than a warp takes are
+    // the block's, before the FP64 work on them.
+    if (n_screen > 0) {
+        const int n_src = shfl_i(rec.i, REC_N);
+        if (n_src >= kWarpEarly) {
+            const int near = __reduce_add_sync(all, lane < n_screen ? b.agg_n[W.scr_slot[lane]] : 0);
+            if (float(n_src) * float(near) > float(WS::kPairs)) return false;
+        }
     }
     o.scanned = total;
     o.status = ST_OK;
