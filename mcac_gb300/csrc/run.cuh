@@ -127,7 +127,7 @@ struct WarpMergeScratch {
     unsigned short pair[496];  // i << 8 | j
 };
 
-constexpr int kMissRun = 4;          // loop_query (step.cuh)
+constexpr int kMissRun = 16;         // loop_query (step.cuh)
 constexpr int kRoundMax = 7;         // steps of a round at most (step.cuh)
 constexpr int kRoundLook = 16;       // rounds between two looks at their pace
 constexpr int kRoundAlone = 64;      // steps one after another that measure theirs

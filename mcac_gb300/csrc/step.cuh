@@ -477,20 +477,22 @@ __device__ __forceinline__ WarpPicked warp_pick(LS &sm, int rnd) {
 
 // warp_query on the scratch of the round's step k. Where the last kMissRun
 // queries of larger aggregates were the block's (dense boxes of few aggregates),
-// the next ones go there without a try, all but every sixteenth.
+// the next ones go there without a try, all but every eighth. (64 boxes of 200
+// spheres in 8 aggregates at 8000 ppm, 600 steps on 128 threads: 12.9 -> 12.3
+// ms; after a run of 4, boxes of 100 aggregates of a few spheres lost 4%.)
 template <class LS>
 __device__ __forceinline__ bool loop_query(LS &sm, int k, int src, const WarpRec &rec, double dl, double full,
                                            WarpAnswer &o) {
     const int *live = sm.live.on ? sm.live.slot : nullptr;
     const bool large = shfl_i(rec.i, REC_N) >= kWarpEarly;
     bool ok = false;
-    if (!large || sm.misses < kMissRun || (sm.misses & 15) == 0) {
+    if (!large || sm.misses < kMissRun || (sm.misses & 7) == 0) {
         if constexpr (LS::kRounds > 1)
             ok = warp_query(sm.R.box, &sm.sc, sm.u.r[k], live, sm.live.n, src, rec, dl, full, o);
         else
             ok = warp_query(sm.R.box, &sm.sc, sm.u.w, live, sm.live.n, src, rec, dl, full, o);
     }
-    if (large && k == 0) {
+    if (large && k == 0 && (!ok || sm.misses != 0)) {
         __syncwarp();
         if ((threadIdx.x & 31) == 0) sm.misses = ok ? 0 : sm.misses + 1;
         __syncwarp();
@@ -1066,6 +1068,7 @@ __device__ inline void rounds_decide(LS &sm, unsigned t_start) {
 template <class LS>
 __device__ inline void rounds_count(LS &sm) {
     const int lane = threadIdx.x & 31, c = sm.n_commit;
+    if (c < 2) return;
     const DevBox &b = sm.R.box;
     int pj = 1;  // pairs as in rounds_decide
     while (lane >= (pj * (pj + 1)) / 2) ++pj;
@@ -1080,8 +1083,11 @@ __device__ inline void rounds_count(LS &sm) {
         };
         auto verlet = [&](int key) { return in(key & 1023, (key >> 10) & 1023, key >> 20, b.n_div); };
         auto fine = [&](int cell) {
-            const int n = b.fine_div, row = cell / n;
-            return in(row / n, row % n, cell % n, n);
+            // quotients by an FP32 reciprocal: exact below 2^21 cells
+            const int n = b.fine_div;
+            const float inv = 1.f / float(n);
+            const int row = int((float(cell) + 0.5f) * inv), i = int((float(row) + 0.5f) * inv);
+            return in(i, row - i * n, cell - row * n, n);
         };
         if (y.axis[0].y & kFineLists) {
             if (x.fine != x.old_fine) listed = fine(x.fine) - fine(x.old_fine);
@@ -1089,6 +1095,7 @@ __device__ inline void rounds_count(LS &sm) {
             listed = verlet(x.key) - verlet(x.old_key);
         }
     }
+    if (!__any_sync(0xffffffffu, listed != 0)) return;
     listed = __reduce_add_sync(0xffffffffu, listed);
     if (lane == 0 && sm.R.lim.with_collisions) sm.st.c_scanned += listed;
 }

@@ -2,7 +2,7 @@
 
 Dense boxes of few aggregates: a warp counts a query's pairs before its FP64
 filter and leaves it early, and after some such queries in a row the next ones
-go to the block without a try, all but every sixteenth. Runs must have the
+go to the block without a try, all but every eighth. Runs must have the
 bits of the block's own steps, with sources on both sides of the size from
 which this holds (8 spheres) and the small and the large mixed.
 """
