@@ -692,15 +692,21 @@ int BatchRunner::set_threads(int threads) {
 // box's step is a chain of dependent loads and block barriers whose parallel
 // parts (the neighbour scan, the sphere-pair search, the merge's pair
 // search) shorten with more threads; a second wave of blocks, though, would
-// wait for the first (and time-capped launches give each block its budget
-// from its own start, so a second wave also halves every box's share of a
-// launch). Timing a few steps of each size, as this once did, chose by the
-// boxes' cheap first steps and, late in a run, spent seconds on steps of the
-// large aggregates run with 32 threads. Speculative rounds (spec.cuh) stay
-// off unless set (set_speculation): clusters of several blocks per box
-// leave fewer boxes resident at a given block size, and measured on the
-// benchmark ensemble they gained at most 10% on its slowest chains. Returns
-// ST_OK (nothing is run).
+// wait for the first. Kernel ms of one launch on 512 boxes of 256 to 16 384
+// monomers: the first 4000 steps 132 / 94 / 85 / 98 / 120 at 32 / 64 / 128 /
+// 256 / 512 threads (the rule takes 128), the first 20 000 4336 / 1657 / 958 /
+// 588 / 493; 304 boxes: 120 / 84 / 73 / 78 / 94 (it takes 256) and 4280 / 1617 /
+// 916 / 560 / 411; 152 boxes: 92 / 65 / 64 / 68 / 69 (it takes 512) and 3440 /
+// 1204 / 713 / 454 / 369. So a long launch of large aggregates would be faster
+// in two waves of larger blocks, which the rule does not look for (time-capped
+// launches give each block its budget from its own start, so a second wave
+// also halves every box's share of a launch). Timing a few steps of each size,
+// as this once did, chose by the boxes' cheap first steps and, late in a run,
+// spent seconds on steps of the large aggregates run with 32 threads.
+// Speculative rounds (spec.cuh) stay off unless set (set_speculation):
+// clusters of several blocks per box leave fewer boxes resident at a given
+// block size, and measured on the benchmark ensemble they gained at most 10%
+// on its slowest chains. Returns ST_OK (nothing is run).
 int BatchRunner::tune(int64_t, int64_t *, float *, std::string *err, bool) {
     if (!auto_threads_ && threads_ != 0) return ST_OK;
     int best = kRunThreadChoices[0];

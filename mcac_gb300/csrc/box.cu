@@ -989,11 +989,13 @@ class CopyStreams {
     cudaEvent_t ev_ = nullptr;
 };
 constexpr int kCopyStreams = 4;
-// one kernel's copies (k_copy_pieces) from this many boxes on (below, the few
-// copies cost less than its table), of less than this many bytes of device
-// memory each (above, the 2 us a copy do not matter and the copy engines
-// leave the SMs free)
-constexpr int kPieceMinBoxes = 16;
+// one kernel's copies (k_copy_pieces) from two boxes on (one box has five
+// copies; load + store in ms, by the driver's copies / by the kernel: 2 boxes
+// of 500 spheres 0.44 + 0.15 / 0.36 + 0.11, 8 of them 1.06 + 0.24 / 0.94 + 0.14,
+// 64 of them 2.31 + 0.84 / 1.74 + 0.30, 200 of 5000 spheres 5.9 + 4.5 / 3.0 +
+// 2.5), of less than this many bytes of device memory each (above, the 2 us a
+// copy do not matter and the copy engines leave the SMs free)
+constexpr int kPieceMinBoxes = 2;
 constexpr size_t kPieceMaxBox = size_t(64) << 20;
 
 }  // namespace

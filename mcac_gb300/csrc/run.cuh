@@ -128,6 +128,13 @@ struct WarpMergeScratch {
 };
 
 constexpr int kMissRun = 16;         // loop_query (step.cuh)
+// The choice between rounds and steps one after another (block_rounds), kernel
+// ms on 32 boxes of 1000 monomers / 152 boxes of 4000 / 152 late boxes / 300
+// boxes of 60 aggregates: 28.2 / 31.8 / 5.5 / 22.4 with these; 35.8 / 46.8 /
+// 5.3 / 21.3 with a quarter of Look and Alone (too short to tell the two
+// apart), 28.9 / 31.2 / 6.0 / 24.3 with four times them; 28.2 / 29.9 / 5.7 /
+// 23.0 with a quarter of Back and BackMax, 28.2 / 42.9 / 5.5 / 21.7 with four
+// times them; Again at 8: 30.8 / 33.6 / 5.5 / 22.3, at 512 within noise.
 constexpr int kRoundMax = 7;         // steps of a round at most (step.cuh)
 constexpr int kRoundLook = 16;       // rounds between two looks at their pace
 constexpr int kRoundAlone = 64;      // steps one after another that measure theirs
