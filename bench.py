@@ -149,21 +149,20 @@ def query_bytes(prof: dict) -> float:
 
 
 # DRAM bytes per MC step of the batched loop on this machine, from one ncu
-# capture of k_run (8 replicas x 200 steps, 32 threads per box): 10.76 MB
-# read + 768 B written over 1,600 steps. The full-size launch (2432 boxes,
-# ~185 GB) is too large to capture; its traffic grows with the steps done.
-K_RUN_DRAM_BYTES_PER_STEP = 6.72e3
+# capture of k_run (304 replicas x 2000 steps, 32 threads per box, 1-pass
+# metrics): 5.48 GB read + 0.38 GB written over 608,000 steps.
+K_RUN_DRAM_BYTES_PER_STEP = 9.63e3
 # DRAM bytes of one k_query_batch launch of the contact-search workload
 # (10,000 queries on the 1,000,000-sphere snapshot), from one ncu capture.
-K_QUERY_BATCH_DRAM_BYTES = 12.12e6
+K_QUERY_BATCH_DRAM_BYTES = 12.49e6
 # DRAM bytes per MC step of k_run on the ensemble benchmark's window a, from
 # one ncu capture of the full-size benchmark (1-pass metrics
-# dram__bytes_read.sum + dram__bytes_write.sum, window a's launch: 72.1 GB
-# read + 13.1 GB written over 18.15 M steps in 2.94 s). A small case of the
-# same kernel that stays in L2 moves 1.28 kB per step.
-K_RUN_ENS_DRAM_BYTES_PER_STEP = 4.69e3
+# dram__bytes_read.sum + dram__bytes_write.sum, window a's launch: 100.8 GB
+# read + 14.3 GB written over 18.15 M steps in 1.65 s). A small case of the
+# same kernel (128 boxes) moves 1.92 kB per step.
+K_RUN_ENS_DRAM_BYTES_PER_STEP = 6.34e3
 K_RUN_ENS_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum (1 pass) of window a's k_run launch of "
-                            "this benchmark at full size: 85.2 GB over 18.15 M MC steps, 4.69 kB per step, scaled "
+                            "this benchmark at full size: 115.1 GB over 18.15 M MC steps, 6.34 kB per step, scaled "
                             "by the MC steps of one launch (window b's launch moves less per step)")
 
 
@@ -346,7 +345,7 @@ def run_ours(args, rank: int, world: int) -> dict | None:
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_kind": peak_kind, "traffic": K_RUN_DRAM_BYTES_PER_STEP * steps_all / max(1, launches),
                      "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one k_run launch on "
-                                       "8 replicas x 200 steps (32 threads per box), 6.7 kB per MC step, scaled "
+                                       "304 replicas x 2000 steps (32 threads per box), 9.6 kB per MC step, scaled "
                                        "by the MC steps of one launch",
                      "kernel": "k_run (batched MC loop)",
                      "bytes_per_launch": qbytes / max(1, launches), "us_per_launch": 1000.0 * total_ms / max(1, launches),
@@ -447,7 +446,7 @@ def run_contact_search(args, rank: int, world: int) -> dict | None:
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_kind": peak_kind, "traffic": K_QUERY_BATCH_DRAM_BYTES,
                      "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one k_query_batch "
-                                       "launch of this workload (9.90 MB + 0.71 MB)",
+                                       "launch of this workload (10.39 MB + 2.10 MB)",
                      "kernel": "k_query_batch",
                      "bytes_per_launch": qbytes / max(1, args.steps),
                      "us_per_launch": 1000.0 * total_ms / max(1, args.steps),

@@ -164,8 +164,8 @@ typedef struct mcacg_profile {
     int64_t queries, merges, translates;
     double query_ms, merge_ms;
     int64_t mov_spheres;  /* spheres of the moving aggregates */
-    int64_t scanned;      /* aggregates read from the Verlet cells */
-    int64_t cells;        /* Verlet cells scanned */
+    int64_t scanned;      /* aggregates read from the cells, or from the live list once few are left */
+    int64_t cells;        /* cells scanned (none with the live list) */
     int64_t candidates;   /* aggregates passing the bounding-sphere filter */
     int64_t cand_spheres; /* spheres of those candidates */
     int64_t refined;      /* sphere pairs evaluated in FP64 */
@@ -247,7 +247,7 @@ int mcacg_box_set_time(mcacg_box *box, double time);
 int mcacg_distance_to_next_contact(mcacg_box *box, int64_t source, const double direction[3], double distance,
                                    mcacg_contact *out);
 /* n independent AggregatList::distance_to_next_contact queries on the
- * current state, run concurrently on the GPU (one thread block per query):
+ * current state, run concurrently on the GPU (a warp or a thread block per query):
  * sources[k], directions[3k..3k+2], distances[k] -> out[k]. Nothing is
  * moved; each result is that of mcacg_distance_to_next_contact on the same
  * state. kernel_ms (may be NULL) receives the kernel's GPU time. No
