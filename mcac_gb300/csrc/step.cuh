@@ -485,16 +485,18 @@ __device__ __forceinline__ bool loop_query(LS &sm, int k, int src, const WarpRec
                                            WarpAnswer &o) {
     const int *live = sm.live.on ? sm.live.slot : nullptr;
     const bool large = shfl_i(rec.i, REC_N) >= kWarpEarly;
+    // (warp 0 alone reads and writes its count while a round is under way)
+    const int missed = k == 0 ? sm.misses : sm.round_misses;
     bool ok = false;
-    if (!large || sm.misses < kMissRun || (sm.misses & 7) == 0) {
+    if (!large || missed < kMissRun || (missed & 7) == 0) {
         if constexpr (LS::kRounds > 1)
             ok = warp_query(sm.R.box, &sm.sc, sm.u.r[k], live, sm.live.n, src, rec, dl, full, o);
         else
             ok = warp_query(sm.R.box, &sm.sc, sm.u.w, live, sm.live.n, src, rec, dl, full, o);
     }
-    if (large && k == 0 && (!ok || sm.misses != 0)) {
+    if (large && k == 0 && (!ok || missed != 0)) {
         __syncwarp();
-        if ((threadIdx.x & 31) == 0) sm.misses = ok ? 0 : sm.misses + 1;
+        if ((threadIdx.x & 31) == 0) sm.misses = ok ? 0 : missed + 1;
         __syncwarp();
     }
     return ok;
@@ -858,7 +860,8 @@ struct LoopSmemT : RS {
     RunState st;
     DevScalars sc;
     long long left;  // steps still allowed in this launch
-    int misses;      // queries of larger aggregates in a row that were the block's (loop_query)
+    int misses;      // queries of larger aggregates in a row that were the block's (loop_query),
+    int round_misses;  // and as they were at the round's start
     int far;         // block_op: the query's aggregate is the block's to move
     const int *rec_ptr[REC_INTS];  // the integer tables of a slot's record
 };
@@ -1166,6 +1169,7 @@ __device__ inline void block_rounds(LS &sm, long long max_steps) {
                 }
                 if (st.finished || st.status != ST_OK || sm.stop) k = 0;
                 if (k > 0 && sm.deadline != 0ULL && global_ns() >= sm.deadline) k = 0;
+                sm.round_misses = sm.misses;
                 sm.n_jobs = k > 0 && sm.seq > 0 ? -1 : k;  // -1: warp 0 alone
             }
             __syncthreads();
